@@ -1,0 +1,49 @@
+"""Many-row products of the layered sequence engine (bf16 mode, CTA pairs on tcgen05) at the edges of their tiles: row counts around 128 and
+256, column counts that are no multiple of a tile, of 32 or of 4, inner sizes that end inside a k-step, activated columns that start off a
+16-byte boundary.  Against the plain float64 implementation."""
+import numpy as np
+import pytest
+
+import binusun_cases
+import binusun_plain
+import nubipel_cases
+import nubipel_plain
+
+pytestmark = pytest.mark.gpu
+
+# every product rounds its rows to bf16 (2^-9 of a value); a dozen such roundings in a row, largest error over the largest logit
+TOL = 12 * 2.0 ** -9
+
+
+def one_step(m, toks):
+    s = m.open()
+    out = m.step([(s, toks)], [range(len(toks))])
+    m.close(s)
+    return out
+
+
+@pytest.mark.parametrize("rows", [33, 64, 127, 128, 129, 255, 256, 257, 520])
+@pytest.mark.parametrize("width,ff,vocab", [(72, 328, 133), (264, 1000, 300), (64, 64, 64)])
+def test_rows_and_columns_around_tiles(rows, width, ff, vocab):
+    cfg = binusun_cases.make_config([binusun_cases.attn_layer(heads=3, kv_heads=1, dim=40, vdim=24, rot_dims=8, window=50, ff=ff)], vocab=vocab, width=width)
+    W = binusun_cases.random_weights(cfg, seed=rows)
+    toks = [int(t) for t in np.random.default_rng(rows).integers(0, vocab, rows)]
+    m = binusun_cases.build_engine(cfg, W, "bfloat16")
+    got = one_step(m, toks)
+    m.free()
+    want = binusun_plain.forward(cfg, W, toks)
+    assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+
+
+@pytest.mark.parametrize("rows", [40, 200, 257])
+@pytest.mark.parametrize("heads,ff", [(4, 64), (3, 72), (5, 200)])   # q, k, v columns in front of the activated ones: 176, 132, 220
+def test_activated_columns(rows, heads, ff):
+    cfg = nubipel_cases.make_config([nubipel_cases.attn(heads=heads, kv_heads=1, dim=12, vdim=20, chunk=24, mlp=nubipel_cases.dense(ff)),
+                                     nubipel_cases.latent(mlp=nubipel_cases.dense(ff))], width=136, vocab=140)
+    W = nubipel_cases.random_weights(cfg, seed=rows + ff)
+    toks = [int(t) for t in np.random.default_rng(rows).integers(0, cfg["vocab"], rows)]
+    m = nubipel_cases.build_engine(cfg, W, "bfloat16")
+    got = one_step(m, toks)
+    m.free()
+    want, _ = nubipel_plain.run(cfg, W, toks)
+    assert np.abs(got - want).max() <= TOL * np.abs(want).max()

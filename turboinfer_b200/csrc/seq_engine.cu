@@ -672,10 +672,10 @@ __global__ void add_one_kernel(float* w, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) w[i] += 1.f;
 }
 
-// ---- tensor maps for the tcgen05 path: a bf16 matrix [rows][cols], cols contiguous, boxes of 64 x 128 with the 128-byte swizzle ----
+// ---- tensor maps for the tcgen05 path: a bf16 matrix [rows][cols], cols contiguous, boxes of 64 x box_rows with the 128-byte swizzle ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t pitch) {   // pitch: elements between rows
+int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t pitch, int box_rows) {   // pitch: elements between rows
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
         void* p = nullptr;
@@ -686,7 +686,7 @@ int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t cols, uint64_t r
     }
     const cuuint64_t dims[2] = {cols, rows};
     const cuuint64_t strides[1] = {pitch * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kSgBK, (cuuint32_t)kSgBM};
+    const cuuint32_t box[2] = {(cuuint32_t)kSgBK, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -733,12 +733,17 @@ bool tc_ok(const Model& m, const void* W, int M, int N, int K) {
 int gemm_tc(Model& m, const __nv_bfloat16* A, int lda, const void* W, float* C, int ldc, int M, int N, int K, int epi = EPI_NONE, float alpha = 1.f, float beta = 0.f,
             const GluCols* cols = nullptr) {
     CUtensorMap ma, mw;
-    TRY(make_tmap_bf16(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda));
-    TRY(make_tmap_bf16(&mw, W, (uint64_t)K, (uint64_t)N, (uint64_t)K));
-    TcArgs g{};
+    PairArgs p{};
+    const int pairs = g_num_sms / 2;
+    p.bn = pair_tile_columns(M, N, K, pairs);
+    p.tiles_m = (M + 255) / 256;
+    p.tiles = p.tiles_m * ((N + p.bn - 1) / p.bn);
+    TRY(make_tmap_bf16(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, kSgBM));
+    TRY(make_tmap_bf16(&mw, W, (uint64_t)K, (uint64_t)N, (uint64_t)K, p.bn / 2));
+    TcArgs& g = p.t;
     g.M = M; g.N = N; g.K = K; g.C = C; g.ldc = ldc; g.epi = epi; g.alpha = alpha; g.beta = beta; g.err = m.err.p;
     if (cols) g.cols = *cols;
-    gemm_bf16_tc_kernel<<<dim3((N + kSgBN - 1) / kSgBN, (M + kSgBM - 1) / kSgBM), kSgThreads, kSgSmemBytes, g_stream>>>(ma, mw, g);
+    TRY(launch_dep(gemm_bf16_tc_kernel, dim3(2 * std::min(p.tiles, pairs)), dim3(kSgThreads), kSgSmemBytes, ma, mw, p));
     LAUNCHED();
     return 0;
 }
