@@ -52,3 +52,18 @@ def test_gemm_asymmetric_and_zero_rows(tb, port):
             qw.free()
         assert np.array_equal(y[[0, 5, 63]], yv)
         assert not y[5].any()
+
+
+@pytest.mark.parametrize("qt", [oracle.QINT4, oracle.QINT8])
+@pytest.mark.parametrize("M", [31, 33, 95, 97, 159, 161, 321])     # tiles of 32 .. 160 tokens, cut anywhere
+@pytest.mark.parametrize("K,N", [(100, 129), (384, 255), (640, 4)])   # columns of a pair's tile: 256, 128 a CTA
+def test_gemm_every_row_equals_gemv_at_tile_edges(tb, qt, M, K, N):
+    rng = np.random.default_rng(M * K + N)
+    w = rng.uniform(-1.0, 1.0, (K, N)).astype(np.float32)
+    x = (rng.standard_normal((M, K)) * np.exp(rng.uniform(-3, 3, (M, 1)))).astype(np.float32)
+    qw = tb.QWeight(w, qt)
+    try:
+        y, yv = qw.gemm(x), qw.gemv(x)
+    finally:
+        qw.free()
+    assert np.array_equal(y, yv)

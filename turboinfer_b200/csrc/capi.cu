@@ -139,6 +139,19 @@ int pick_stages(const QLayout& L, int* stages, size_t* smem) {
     return fail("GEMV K=%d does not fit shared memory (x digits need %d KiB)", L.K, layout_kpad(L) * 3 / 1024);
 }
 
+// A tensor-core GEMM whose bounded waits ran out leaves a 1 in this mapped host word (its results are then not to be used); read behind
+// every synchronisation of the library stream.
+int* g_gemm_err = nullptr;
+int* g_gemm_err_dev = nullptr;
+int sync_stream() {
+    CK(cudaStreamSynchronize(g_stream));
+    if (g_gemm_err && *reinterpret_cast<volatile int*>(g_gemm_err)) {
+        *reinterpret_cast<volatile int*>(g_gemm_err) = 0;
+        return fail("a tensor-core GEMM gave up waiting for its operands");
+    }
+    return 0;
+}
+
 int set_kernel_attrs() {
     // every cudaFuncSetAttribute of the library in one place, behind one flag that ti_b200_shutdown resets: attributes
     // belong to the device context, so a fresh init (same or another device) must set them again
@@ -289,7 +302,7 @@ int build_qweight_views(const SrcView* v, int nsrc, int mode, int K, int qtype, 
     CK(cudaGetLastError());
     float h[6] = {0};
     CK(cudaMemcpyAsync(h, sz.p, sizeof(float) * 2 * nsrc, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     w->scale = h[0];
     w->zp = h[1];
     w->has_zterm = false;
@@ -449,7 +462,7 @@ Model* get_model(ti_model_t h) {
 int upload(DevBuf<float>& dst, const float* host, size_t n) {
     TRY(dst.alloc(n));
     CK(cudaMemcpyAsync(dst.p, host, n * sizeof(float), cudaMemcpyHostToDevice, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -773,7 +786,7 @@ int tp_exchange_setup(Model& m) {
     if (r != ncclSuccess) return fail("ncclAllGather (IPC handles) failed: %s", g_nccl.GetErrorString(r));
     std::vector<cudaIpcMemHandle_t> all(P);
     CK(cudaMemcpyAsync(all.data(), hrecv.p, sizeof(mine) * P, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     for (int q = 0; q < P; ++q) {
         if (q == m.tp_rank) { m.peer_base[q] = m.xchg; continue; }
         const cudaError_t e = cudaIpcOpenMemHandle(&m.peer_base[q], all[q], cudaIpcMemLazyEnablePeerAccess);
@@ -782,7 +795,7 @@ int tp_exchange_setup(Model& m) {
     // nobody may signal a block that its owner has not zeroed yet: one more collective as a barrier
     const ncclResult_t r2 = g_nccl.AllGather(hsend.p, hrecv.p, sizeof(mine), ncclUint8, g_comm, g_stream);
     if (r2 != ncclSuccess) return fail("ncclAllGather (barrier) failed: %s", g_nccl.GetErrorString(r2));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -976,7 +989,7 @@ int build_mega(Model& m) {
     }
     TRY(m.prod.alloc(prod.size()));
     CK(cudaMemcpyAsync(m.prod.p, prod.data(), prod.size() * sizeof(ProdRec), cudaMemcpyHostToDevice, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     TRY(m.emb_stats.alloc(m.cfg.vocab));
     emb_stats_kernel<<<m.cfg.vocab, 256, 0, g_stream>>>(m.tok_emb.p, m.layers.empty() ? m.out_norm.p : m.layers[0].attn_norm.p,
                                                         m.emb_stats.p, H);
@@ -986,7 +999,7 @@ int build_mega(Model& m) {
     TRY(m.head_cnt.alloc(std::max(1, m.attn_heads)));
     CK(cudaMemsetAsync(m.sync_buf.p, 0, (kBarWords * kBarStride + 8) * sizeof(unsigned int), g_stream));
     CK(cudaMemsetAsync(m.head_cnt.p, 0, std::max(1, m.attn_heads) * sizeof(unsigned int), g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     int bits = m.cfg.qtype == TI_Q_INT4 ? 4 : 8;
     int per_sm = 0;
     if (bits == 4) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mega_decode_kernel<4>, kMegaThreads, m.mega_smem));
@@ -1058,7 +1071,7 @@ int run_mega(Model& m, int n_prompt, int n_steps, int first_sample) {
 // ---- tensor-core GEMM (prefill / batched decode) ---------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int make_tmap_u8_2d(CUtensorMap* map, void* base, uint64_t cols, uint64_t rows, int box_rows = kGemmBM) {
+int make_tmap_u8(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
         void* p = nullptr;
@@ -1067,12 +1080,9 @@ int make_tmap_u8_2d(CUtensorMap* map, void* base, uint64_t cols, uint64_t rows, 
         if (!p || qr != cudaDriverEntryPointSuccess) return fail("cuTensorMapEncodeTiled is not available in this driver");
         fn = reinterpret_cast<EncodeTiledFn>(p);
     }
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols};          // bytes between rows
-    const cuuint32_t box[2] = {(cuuint32_t)kGemmBK, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed (%d)", (int)r);
     return 0;
 }
@@ -1086,51 +1096,6 @@ int ensure_kmajor(QWeight& w) {
     unpack_kmajor_kernel<<<w.L.P, kConsumerThreads, 0, g_stream>>>(w.packed.p, w.L, w.k_pad, w.kmajor.p);
     ++g_launches;
     CK(cudaGetLastError());
-    return 0;
-}
-
-// x_dev [M][K] fp32 -> y_dev [M][N] fp32; scratch buffers are allocated per call (this entry point is not the decode path)
-int gemm_q_dev(QWeight& w, const float* x_dev, float* y_dev, int M, float* kernel_ms, int reps) {
-    TRY(ensure_kmajor(w));
-    const int K = w.L.K, N = w.L.N;
-    const int m_pad = (M + kGemmBM - 1) / kGemmBM * kGemmBM;
-    DevBuf<int8_t> planes;
-    DevBuf<float> sx;
-    DevBuf<long long> sxf;
-    TRY(planes.alloc((size_t)3 * m_pad * w.k_pad));
-    TRY(sx.alloc(M));
-    TRY(sxf.alloc(M));
-    CK(cudaMemsetAsync(planes.p, 0, (size_t)3 * m_pad * w.k_pad, g_stream));
-    gemm_digits_kernel<<<M, 256, 0, g_stream>>>(x_dev, M, K, m_pad, w.k_pad, planes.p, sx.p, sxf.p);
-    ++g_launches;
-    CK(cudaGetLastError());
-    CUtensorMap map_a;
-    TRY(make_tmap_u8_2d(&map_a, planes.p, (uint64_t)w.k_pad, (uint64_t)3 * m_pad));
-    GemmArgs g{};
-    g.M = M; g.N = N; g.K = K;
-    g.m_pad = m_pad; g.k_pad = w.k_pad;
-    g.a_signed_b = w.L.bits == 8 ? 1 : 0;
-    g.woff = w.L.bits == 4 ? w.offset4 : 0;
-    g.sx = sx.p; g.sxf = sxf.p;
-    g.colscale = w.colscale.p;
-    g.colzterm = w.has_zterm ? w.colzterm.p : nullptr;
-    g.y = y_dev;
-    g.wt = w.kmajor.p;
-    const dim3 grid((N + kGemmBN - 1) / kGemmBN, m_pad / kGemmBM);
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (kernel_ms) { CK(cudaEventCreate(&e0)); CK(cudaEventCreate(&e1)); CK(cudaEventRecord(e0, g_stream)); }
-    for (int r = 0; r < std::max(reps, 1); ++r) {
-        gemm_i8_tc_kernel<<<grid, kGemmThreads, kGemmSmemBytes, g_stream>>>(map_a, g);
-        ++g_launches;
-    }
-    CK(cudaGetLastError());
-    if (kernel_ms) CK(cudaEventRecord(e1, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
-    if (kernel_ms) {
-        CK(cudaEventElapsedTime(kernel_ms, e0, e1));
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-    }
     return 0;
 }
 
@@ -1152,6 +1117,68 @@ int launch_step(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args
     cfg.numAttrs = g_batch_pdl ? 1 : 0;
     CK(cudaLaunchKernelEx(&cfg, kern, KArgs(args)...));
     ++g_launches;
+    return 0;
+}
+
+// the tensor-core GEMM of many rows (gemm_tc.cuh): tensor maps over the digit planes and the weights' tile images, tile width
+struct PairLaunch { CUtensorMap x, w; PairGemmArgs a; int pairs; };
+int pair_gemm_setup(const QWeight& w, const int8_t* planes, const GemmArgs& g, PairLaunch* out) {
+    const int n_tiles = (g.N + 2 * kGemmBN - 1) / (2 * kGemmBN), KB = g.k_pad / kGemmBK, pairs = g_num_sms / 2;
+    out->a = PairGemmArgs{g, i8_tile_tokens(g.M, n_tiles, KB, pairs), 0, 0, g_gemm_err_dev};
+    out->a.tiles_t = (g.M + out->a.T - 1) / out->a.T;
+    out->a.tiles = out->a.tiles_t * n_tiles;
+    out->pairs = std::min(out->a.tiles, pairs);
+    const cuuint64_t xd[3] = {(cuuint64_t)g.k_pad, (cuuint64_t)g.M, 3}, xs[2] = {(cuuint64_t)g.k_pad, (cuuint64_t)g.m_pad * g.k_pad};
+    const cuuint32_t xb[3] = {(cuuint32_t)kGemmBK, (cuuint32_t)out->a.T / 2, 3};
+    TRY(make_tmap_u8(&out->x, planes, 3, xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_128B));
+    const cuuint64_t wd[2] = {(cuuint64_t)kGemmBK, (cuuint64_t)w.n_pad * KB}, ws[1] = {(cuuint64_t)kGemmBK};   // (the images are swizzled already)
+    const cuuint32_t wb[2] = {(cuuint32_t)kGemmBK, (cuuint32_t)kGemmBN};
+    return make_tmap_u8(&out->w, w.kmajor.p, 2, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+int pair_gemm_launch(const PairLaunch& p) {
+    return launch_step(gemm_i8_tc_kernel, dim3(2 * p.pairs), dim3(kGemmThreads), kGemmSmemBytes, p.x, p.w, p.a);
+}
+
+// x_dev [M][K] fp32 -> y_dev [M][N] fp32; scratch buffers are allocated per call (this entry point is not the decode path)
+int gemm_q_dev(QWeight& w, const float* x_dev, float* y_dev, int M, float* kernel_ms, int reps) {
+    TRY(ensure_kmajor(w));
+    const int K = w.L.K, N = w.L.N;
+    const int m_pad = (M + kGemmBM - 1) / kGemmBM * kGemmBM;
+    DevBuf<int8_t> planes;
+    DevBuf<float> sx;
+    DevBuf<long long> sxf;
+    TRY(planes.alloc((size_t)3 * m_pad * w.k_pad));
+    TRY(sx.alloc(M));
+    TRY(sxf.alloc(M));
+    CK(cudaMemsetAsync(planes.p, 0, (size_t)3 * m_pad * w.k_pad, g_stream));
+    gemm_digits_kernel<<<M, 256, 0, g_stream>>>(x_dev, M, K, m_pad, w.k_pad, planes.p, sx.p, sxf.p);
+    ++g_launches;
+    CK(cudaGetLastError());
+    GemmArgs g{};
+    g.M = M; g.N = N; g.K = K;
+    g.m_pad = m_pad; g.k_pad = w.k_pad;
+    g.a_signed_b = w.L.bits == 8 ? 1 : 0;
+    g.woff = w.L.bits == 4 ? w.offset4 : 0;
+    g.sx = sx.p; g.sxf = sxf.p;
+    g.colscale = w.colscale.p;
+    g.colzterm = w.has_zterm ? w.colzterm.p : nullptr;
+    g.y = y_dev;
+    g.wt = w.kmajor.p;
+    PairLaunch pl;
+    TRY(pair_gemm_setup(w, planes.p, g, &pl));
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    if (kernel_ms) { CK(cudaEventCreate(&e0)); CK(cudaEventCreate(&e1)); CK(cudaEventRecord(e0, g_stream)); }
+    for (int r = 0; r < std::max(reps, 1); ++r) {
+        TRY(pair_gemm_launch(pl));
+    }
+    CK(cudaGetLastError());
+    if (kernel_ms) CK(cudaEventRecord(e1, g_stream));
+    TRY(sync_stream());
+    if (kernel_ms) {
+        CK(cudaEventElapsedTime(kernel_ms, e0, e1));
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+    }
     return 0;
 }
 
@@ -1195,13 +1222,9 @@ int pf_gemm(Model& m, QWeight& w, int M, int m_pad, float* y, const float* resid
         CK(cudaGetLastError());
         return 0;
     }
-    CUtensorMap map_a;
-    TRY(make_tmap_u8_2d(&map_a, m.pf_planes.p, (uint64_t)w.k_pad, (uint64_t)3 * m_pad));
-    const dim3 grid((w.L.N + kGemmBN - 1) / kGemmBN, m_pad / kGemmBM);
-    gemm_i8_tc_kernel<<<grid, kGemmThreads, kGemmSmemBytes, g_stream>>>(map_a, g);
-    ++g_launches;
-    CK(cudaGetLastError());
-    return 0;
+    PairLaunch pl;
+    TRY(pair_gemm_setup(w, m.pf_planes.p, g, &pl));
+    return pair_gemm_launch(pl);
 }
 // gu != nullptr: x is computed on the fly as up * silu(gate) from gu[M][2K] (needs the fast path; callers check pf_digits_fast)
 bool pf_digits_fast(int K, int k_pad) { return K % 4 == 0 && k_pad <= 4 * kDigitsThreads * kDigitsVecs; }
@@ -1520,7 +1543,7 @@ int literal_quantize(DevBuf<float>& w, int qtype) {
     literal_quant_kernel<<<grid_for(w.n), 256, 0, g_stream>>>(w.p, w.n, qtype, sz.p);
     ++g_launches;
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 int literal_finalize(Model& m) {
@@ -1620,7 +1643,7 @@ int literal_generate(Model& m, int n_prompt, int n_new, int stop_on_eos, int32_t
     int produced = 0, total = n_prompt;
     for (int i = 0; i < n_new; ++i) {
         CK(cudaMemcpyAsync(logits.data(), m.logits.p, (size_t)V * 4, cudaMemcpyDeviceToHost, g_stream));
-        CK(cudaStreamSynchronize(g_stream));
+        TRY(sync_stream());
         if (logits_host) memcpy(logits_host + (size_t)i * V, logits.data(), (size_t)V * 4);
         const int best = literal_pick(logits);
         out_tokens[produced++] = best;
@@ -1630,7 +1653,7 @@ int literal_generate(Model& m, int n_prompt, int n_new, int stop_on_eos, int32_t
         if (i + 1 < n_new) TRY(literal_forward(m, 1));   // decode (:774): one row, position-independent
     }
     CK(cudaEventRecord(e1, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
@@ -1676,6 +1699,11 @@ int ti_b200_init(int device) {
     if (prop.major < 10) return fail("ti_b200_init: device %d is sm_%d%d; this library is built for sm_100a (B200) only", device, prop.major, prop.minor);
     g_num_sms = prop.multiProcessorCount;
     if (!g_stream) CK(cudaStreamCreateWithFlags(&g_stream, cudaStreamNonBlocking));
+    if (!g_gemm_err) {
+        CK(cudaHostAlloc(&g_gemm_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        *g_gemm_err = 0;
+        CK(cudaHostGetDevicePointer(&g_gemm_err_dev, g_gemm_err, 0));
+    }
     g_device = device;
     const char* pdl = getenv("TURBOINFER_B200_PDL");
     g_use_pdl = pdl ? atoi(pdl) != 0 : true;   // programmatic dependent launch of the stand-alone GEMV: on unless TURBOINFER_B200_PDL=0
@@ -1761,7 +1789,7 @@ int ti_b200_tp_init(int nranks, int rank, const uint8_t* unique_id, size_t id_by
 
 int ti_b200_sync(void) {
     TRY(need_init());
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 int ti_b200_malloc(void** dev, size_t bytes) {
@@ -1777,13 +1805,13 @@ int ti_b200_free(void* dev) {
 int ti_b200_memcpy_h2d(void* dev, const void* host, size_t bytes) {
     TRY(need_init());
     CK(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 int ti_b200_memcpy_d2h(void* host, const void* dev, size_t bytes) {
     TRY(need_init());
     CK(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 int ti_b200_launch_count(uint64_t* n) { *n = g_launches; return 0; }
@@ -1801,7 +1829,7 @@ int ti_b200_quant_info(const float* x_host, size_t n, int qtype, int symmetric, 
     TRY(device_quant_params(x.p, n, qtype, symmetric, sz.p, mm.p, g_stream));
     float h[2];
     CK(cudaMemcpyAsync(h, sz.p, sizeof(h), cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     *scale = h[0];
     *zero_point = h[1];
     return 0;
@@ -1821,7 +1849,7 @@ int ti_b200_quantize(const float* x_host, size_t n, int qtype, float scale, floa
     CK(cudaGetLastError());
     if (qtype == TI_Q_INT8) CK(cudaMemcpyAsync(q_out_host, q8.p, n, cudaMemcpyDeviceToHost, g_stream));
     else CK(cudaMemcpyAsync(q_out_host, q32.p, n * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -1844,7 +1872,7 @@ int ti_b200_dequantize(const void* q_host, size_t n, int qtype, float scale, flo
     ++g_launches;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(x_out_host, x.p, n * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -1887,7 +1915,7 @@ int ti_b200_qweight_unpack(ti_qweight_t h, int32_t* q_out_host) {
     ++g_launches;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(q_out_host, q.p, n * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -1921,7 +1949,7 @@ int ti_b200_gemv_q(ti_qweight_t h, const float* x_host, float* y_host, size_t ro
     TRY(y.alloc(rows * N));
     for (size_t r = 0; r < rows; ++r) TRY(ti_b200_gemv_q_dev(h, x.p + r * K, y.p + r * N));
     CK(cudaMemcpyAsync(y_host, y.p, rows * N * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -1935,7 +1963,7 @@ int ti_b200_gemm_q(ti_qweight_t h, const float* x_host, float* y_host, size_t ro
     TRY(y.alloc(rows * w->L.N));
     TRY(gemm_q_dev(*w, x.p, y.p, (int)rows, nullptr, 1));
     CK(cudaMemcpyAsync(y_host, y.p, rows * w->L.N * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -1968,7 +1996,7 @@ int ti_b200_matmul_f32(const float* a_host, const float* b_host, float* c_host, 
     ++g_launches;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(c_host, c.p, M * N * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -1983,7 +2011,7 @@ int ti_b200_rms_norm(const float* x_host, const float* w_host, float* y_host, si
     ++g_launches;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(y_host, y.p, rows * H * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -2011,7 +2039,7 @@ int ti_b200_rope(const float* x_host, const float* pos_host, float* y_host, size
     ++g_launches;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(y_host, y.p, rows * D * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -2026,7 +2054,7 @@ static int elementwise_host(const float* a_host, const float* b_host, float* y_h
     ++g_launches;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(y_host, y.p, n * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 int ti_b200_silu(const float* x, float* y, size_t n) { return elementwise_host(x, nullptr, y, n, EW_SILU); }
@@ -2045,7 +2073,7 @@ int ti_b200_softmax(const float* x_host, float* y_host, size_t rows, size_t n, f
     ++g_launches;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(y_host, y.p, rows * n * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -2108,7 +2136,7 @@ int ti_b200_attention_decode(const float* q_host, const float* k_host, const flo
         CK(cudaGetLastError());
     }
     CK(cudaMemcpyAsync(out_host, out.p, B * H * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -2139,7 +2167,7 @@ int ti_b200_kv_create(int32_t layers, int32_t heads, int32_t head_dim, int32_t m
     kv->max_splits = std::max(1, std::min((2 * g_num_sms + heads - 1) / heads, 512));
     TRY(kv->part_o.alloc((size_t)heads * kv->max_splits * head_dim));
     TRY(kv->part_ml.alloc((size_t)heads * kv->max_splits * 2));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     std::lock_guard<std::mutex> lk(g_mu);
     g_kvs.push_back(std::move(kv));
     *out = g_kvs.size();
@@ -2182,7 +2210,7 @@ int ti_b200_kv_append(ti_kv_t h, int32_t layer, const float* k_new_host, const f
                                                        kv->page_table.p, kv->page_tokens);
     ++g_launches;
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     kv->len[layer] += new_tokens;
     return 0;
 }
@@ -2203,7 +2231,7 @@ int ti_b200_kv_read(ti_kv_t h, int32_t layer, float* k_out_host, float* v_out_ho
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(k_out_host, ko.p, n * 4, cudaMemcpyDeviceToHost, g_stream));
     CK(cudaMemcpyAsync(v_out_host, vo.p, n * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 // attention of one query token over the layer's cached tokens, read in place (flash-decoding, split over the context):
@@ -2243,7 +2271,7 @@ int ti_b200_kv_attention(ti_kv_t h, int32_t layer, const float* q_host, float* o
     g_launches += 2;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out_host, out.p, (size_t)H * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -2295,7 +2323,7 @@ int ti_b200_gemv_q_ex(ti_qweight_t h, const float* x_host, float* y_host, int32_
     a.resid = r.p;
     TRY(launch_gemv(*w, a, g_stream));
     CK(cudaMemcpyAsync(y_host, y.p, n_out * 4, cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -2329,7 +2357,7 @@ int ti_b200_prefill(ti_model_t h, const int32_t* tokens, int32_t n, float* last_
             CK(cudaMemcpyAsync(last_logits_host, m.logits.p, V * 4, cudaMemcpyDeviceToHost, g_stream));
         }
     }
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -2397,7 +2425,7 @@ int ti_b200_model_set_tensor_q(ti_model_t h, const char* name, const void* q_hos
     const size_t bytes = rows * cols * (qtype == TI_Q_INT8 ? 1 : 4);
     TRY(q.qdata.alloc(bytes));
     CK(cudaMemcpyAsync(q.qdata.p, q_host, bytes, cudaMemcpyHostToDevice, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return store_tensor(*m, name, DevBuf<float>(), rows, cols, &q);
 }
 
@@ -2466,7 +2494,7 @@ int ti_b200_model_finalize(ti_model_t h) {
     const int rope_dim = m.cfg.rope_mode == 1 ? H / m.cfg.heads : H;
     std::vector<float> f = host_inv_freq(rope_dim, m.cfg.rope_theta);
     TRY(upload(m.inv_freq, f.data(), f.size()));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     bool complete = true;
     for (auto& ly : m.layers) complete &= (ly.qkv && ly.o && ly.gateup && ly.down);
     const char* eng = getenv("TURBOINFER_B200_ENGINE");
@@ -2571,7 +2599,7 @@ int ti_b200_decode_step(ti_model_t h, int32_t token, float* logits_host, int32_t
         TRY(literal_forward(*m, 1));
         std::vector<float> lg(m->cfg.vocab);
         CK(cudaMemcpyAsync(lg.data(), m->logits.p, lg.size() * 4, cudaMemcpyDeviceToHost, g_stream));
-        CK(cudaStreamSynchronize(g_stream));
+        TRY(sync_stream());
         if (logits_host) memcpy(logits_host, lg.data(), lg.size() * 4);
         if (argmax) *argmax = literal_pick(lg);
         m->host_pos += 1;
@@ -2600,7 +2628,7 @@ int ti_b200_decode_step(ti_model_t h, int32_t token, float* logits_host, int32_t
     }
     int tok = 0;
     CK(cudaMemcpyAsync(&tok, &m->state.p->token, sizeof(int), cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     if (argmax) *argmax = tok;
     return 0;
 }
@@ -2663,7 +2691,7 @@ int ti_b200_generate_greedy(ti_model_t h, const int32_t* prompt, int32_t n_promp
                 steps_done += c;
                 if (steps_done >= n_new - 1) break;
                 CK(cudaMemcpyAsync(seen.data(), m.out_tokens.p, (size_t)(1 + steps_done) * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
-                CK(cudaStreamSynchronize(g_stream));
+                TRY(sync_stream());
                 if (std::find(seen.begin(), seen.begin() + 1 + steps_done, 2) != seen.begin() + 1 + steps_done) break;
             }
         } else {
@@ -2693,7 +2721,7 @@ int ti_b200_generate_greedy(ti_model_t h, const int32_t* prompt, int32_t n_promp
         TRY(gather_sharded_logits(m, m.hist.p, (size_t)have * V));
         CK(cudaMemcpyAsync(logits_host, m.hist.p, (size_t)have * V * 4, cudaMemcpyDeviceToHost, g_stream));
     }
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));
     CK(cudaEventElapsedTime(&m.last_prefill_ms, ep, e0));
@@ -2771,7 +2799,7 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
             for (int p = 0; p < pages; ++p) tab[(size_t)b * pages + p] = b * pages + (pages - 1 - p);   // deliberately not the identity
         TRY(bs.tables.alloc(tab.size()));
         CK(cudaMemcpyAsync(bs.tables.p, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice, g_stream));
-        CK(cudaStreamSynchronize(g_stream));
+        TRY(sync_stream());
         TRY(bs.tokens.alloc(B));
         TRY(bs.lens.alloc(B));
         TRY(bs.pos_step.alloc(2));
@@ -2826,7 +2854,7 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
     CK(cudaEventRecord(e1, g_stream));
     CK(cudaMemcpyAsync(out_tokens, bs.out.p, (size_t)B * n_new * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
     if (logits_last) CK(cudaMemcpyAsync(logits_last, bs.logits.p, (size_t)B * V * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
@@ -2931,7 +2959,7 @@ int ti_b200_beam_search(ti_model_t h, const int32_t* prompt, int32_t n_prompt, i
         TRY(st.v_ptrs.alloc(std::max<size_t>(vp.size(), 1)));
         CK(cudaMemcpyAsync(st.k_ptrs.p, kp.data(), kp.size() * sizeof(float*), cudaMemcpyHostToDevice, g_stream));
         CK(cudaMemcpyAsync(st.v_ptrs.p, vp.data(), vp.size() * sizeof(float*), cudaMemcpyHostToDevice, g_stream));
-        CK(cudaStreamSynchronize(g_stream));
+        TRY(sync_stream());
         TRY(bs.tables.alloc((size_t)B * pages));
         TRY(bs.tokens.alloc(B));
         TRY(bs.pos_step.alloc(2));
@@ -3025,7 +3053,7 @@ int ti_b200_beam_search(ti_model_t h, const int32_t* prompt, int32_t n_prompt, i
         }
         CK(cudaMemcpyAsync(bs.tokens.p, feed.data(), B * sizeof(int), cudaMemcpyHostToDevice, g_stream));
         TRY(run(expand));
-        CK(cudaStreamSynchronize(g_stream));   // tab / pairs / feed are reused by the next step
+        TRY(sync_stream());   // tab / pairs / feed are reused by the next step
         pairs.clear();
         return 0;
     };
@@ -3044,7 +3072,7 @@ int ti_b200_beam_search(ti_model_t h, const int32_t* prompt, int32_t n_prompt, i
         CK(cudaMemcpyAsync(cprob.data(), st.cand_prob.p, cprob.size() * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
         CK(cudaMemcpyAsync(ctok.data(), st.cand_tok.p, ctok.size() * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
         CK(cudaMemcpyAsync(ccnt.data(), st.cand_cnt.p, B * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
-        CK(cudaStreamSynchronize(g_stream));
+        TRY(sync_stream());
         std::vector<Cand> next;
         for (const Cand& c : active) {   // most probable candidate first (the heap order of :1941-1944)
             const int cnt = std::min(ccnt[c.row], B);
@@ -3125,7 +3153,7 @@ int ti_b200_beam_expand(const float* logits_host, size_t rows, size_t vocab, flo
     CK(cudaMemcpyAsync(probs_out, pr.p, rows * beam_size * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
     CK(cudaMemcpyAsync(tokens_out, tk.p, rows * beam_size * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
     CK(cudaMemcpyAsync(counts_out, cn.p, rows * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -3142,7 +3170,7 @@ int ti_b200_sample_logits(const float* logits_host, size_t rows, size_t vocab, f
     TRY(launch_sample(lg.p, (int)rows, (int)vocab, (int)vocab, temperature, top_k, top_p, seed, nullptr, step, tok.p, lp.p, nullptr, nullptr, 0, nullptr));
     CK(cudaMemcpyAsync(tokens_out, tok.p, rows * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
     if (logprobs_out) CK(cudaMemcpyAsync(logprobs_out, lp.p, rows * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -3191,7 +3219,7 @@ int ti_b200_generate_sampled(ti_model_t h, const int32_t* prompt, int32_t n_prom
         if (stop_on_eos && sampled % kEosChunk == 0 && i + 1 < n_new) {   // look at the tokens so far: stop issuing steps after an EOS (:760)
             seen.resize(sampled);
             CK(cudaMemcpyAsync(seen.data(), m.smp_tokens.p, (size_t)sampled * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
-            CK(cudaStreamSynchronize(g_stream));
+            TRY(sync_stream());
             if (std::find(seen.begin(), seen.end(), 2) != seen.end()) break;
         }
         if (i + 1 < n_new) { TRY(decode_pass(m)); ++passes; }
@@ -3204,7 +3232,7 @@ int ti_b200_generate_sampled(ti_model_t h, const int32_t* prompt, int32_t n_prom
         CK(cudaMemcpyAsync(toks.data(), m.smp_tokens.p, sampled * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
         CK(cudaMemcpyAsync(lps.data(), m.smp_logprobs.p, sampled * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
     }
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
@@ -3263,7 +3291,7 @@ int ti_b200_compute_logprobs(ti_model_t h, const int32_t* tokens, int32_t n, flo
     CK(cudaGetLastError());
     m.host_pos = n;
     CK(cudaMemcpyAsync(out, lp.p, n * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     return 0;
 }
 
@@ -3296,7 +3324,7 @@ static int debug_timeline_run(ti_model_t h, int32_t token, int64_t* stamps, size
     TRY(rc);
     m->host_pos += 1;
     CK(cudaMemcpyAsync(stamps, m->dbg.p, want * sizeof(long long), cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     *n_phases = m->nphases;
     if (n_ctas) *n_ctas = g_num_sms;
     return 0;
@@ -3331,7 +3359,7 @@ int ti_b200_bench_gemv(const ti_qweight_t* ws, size_t n_w, size_t reps, float* m
     CK(cudaEventRecord(e0, g_stream));
     for (size_t r = 0; r < reps; ++r) TRY(ti_b200_gemv_q_dev(ws[r % n_w], x.p, y.p));
     CK(cudaEventRecord(e1, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     CK(cudaEventElapsedTime(ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -3371,7 +3399,7 @@ int ti_b200_model_bench_gemv(ti_model_t h, int slot, size_t reps, float* ms, dou
     CK(cudaEventRecord(e0, g_stream));
     for (size_t r = 0; r < reps; ++r) TRY(run(ws[r % ws.size()]));
     CK(cudaEventRecord(e1, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
+    TRY(sync_stream());
     CK(cudaEventElapsedTime(ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

@@ -7,27 +7,35 @@
 // 8-bit digit planes; the tensor cores multiply the INT8 planes with the INT8 / unpacked-INT4 weights (kind::i8, exact
 // int32 accumulation in TMEM, one accumulator per digit); the epilogue recombines the digits in int64 and scales once.
 //
-//   CTA tile      128 tokens x 128 columns, K in steps of 128 bytes; 3 accumulators x 128 columns of TMEM
-//   warp 0        producer: per stage 3 digit tiles of A (TMA boxes of 128 x 128 B, SWIZZLE_128B) + 1 weight tile of B
-//                 (16 KiB, stored in HBM as its swizzled image: one 1-D bulk copy)
-//   warp 1        TMEM allocation; one elected lane issues tcgen05.mma (M 128, N 128, K 32): 4 k-steps x 3 digits per stage,
-//                 tcgen05.commit releases the stage / publishes the accumulators
-//   warps 2..5    epilogue: tcgen05.ld 32x32b (lane = token row), digit recombination, scale, store
+// A pair of neighbouring SMs (cta_group::2) owns a tile of 256 weight columns x T tokens.  The MMA's M side is the weight columns (128 a
+// CTA), its N side the tokens, whose digit rows are split between the two CTAs; D[256 x T] per digit plane, 3 T <= 480 TMEM columns.  A k-step
+// brings 16 KiB of weights and 3 T / 2 digit rows into each CTA for 6 T clocks of tensor work: 48 bytes a clock and SM at T = 160, against
+// 85 for one-CTA tiles of 128 x 128 (L2 gives an SM about 64).  Clusters walk the tiles, tokens fastest.
+//   warp 0        producer: one box of the weights' tile images, one 3-D box of the digit planes (128 B x T / 2 rows x 3 planes,
+//                 SWIZZLE_128B) a stage; both CTAs' copies complete on the even CTA's barrier; 4 stages of 46 KiB
+//   warp 1        TMEM allocation; even CTA: tcgen05.mma (M 256, N T, K 32), 4 k-steps x 3 digits a stage, issued warp-uniformly (elect_one)
+//   warps 2..9    epilogue: tcgen05.ld 32x32b (lane = weight column), digit recombination, scale, residual, stores of 32 neighbouring columns
+// Measured (kernel alone, INT8 weights, B200; before = one-CTA tiles of 128 x 128 with one-lane issue): M 2048, K 4096, N 22016 525 -> 385 us
+// (2.88 POP/s of INT8 work issued), K 4096, N 12288 292 -> 220, K 11008, N 4096 248 -> 184 (3.0 POP/s); M 256, K 4096, N 4096 16 us.  Bound by
+// the tensor pipe at the power cap plus an exposed epilogue of about 3 us a tile.
 // Operands are K-major in shared memory; descriptors follow the sm_100 layout (start address, SBO = 1024 B between 8-row
 // groups, version 1, layout type SWIZZLE_128B); the k-step inside the 128-byte swizzle atom advances the start address.
 #pragma once
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "gemv.cuh"
 
 namespace tib {
 
-constexpr int kGemmBM = 128, kGemmBN = 128, kGemmBK = 128;   // BK in bytes = int8 elements
-constexpr int kGemmStages = 3;
-constexpr int kGemmThreads = 192;
-constexpr int kGemmTileBytes = kGemmBM * kGemmBK;              // 16 KiB
-constexpr int kGemmStageBytes = 4 * kGemmTileBytes;            // 3 A digit tiles + 1 B tile
-constexpr size_t kGemmSmemBytes = (size_t)kGemmStages * kGemmStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int kGemmBM = 128, kGemmBN = 128, kGemmBK = 128;   // row padding of the planes; weight columns of a CTA; BK in bytes = int8 elements
+constexpr int kGemmMaxTokens = 160;
+constexpr int kGemmStages = 4, kGemmEpiWarps = 8;
+constexpr int kGemmThreads = 64 + 32 * kGemmEpiWarps;
+constexpr int kGemmTileBytes = kGemmBN * kGemmBK;              // 16 KiB of weights
+constexpr int kGemmStageBytes = kGemmTileBytes + 3 * (kGemmMaxTokens / 2) * kGemmBK;   // + three digit planes of half the tile's tokens: 46 KiB
+constexpr size_t kGemmSmemBytes = (size_t)kGemmStages * kGemmStageBytes + 1024 /*align*/ + 256 /*barriers*/ + kGemmMaxTokens * 12 /*s_x, sum(xf)*/;
 
 struct GemmArgs {
     int M, N, K;            // logical sizes
@@ -122,6 +130,66 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* err) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (!mbar_try_wait(bar, parity)) {
+        if (clock64() - t0 > 2000000000LL) {   // about a second
+            *reinterpret_cast<volatile int*>(err) = 1;   // (device or mapped host memory)
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the shared-memory address of the even CTA's copy of a barrier (bit 24 of a shared::cluster address is the CTA's place in its pair)
+__device__ __forceinline__ uint32_t pair_leader(uint32_t saddr) { return saddr & 0xFEFFFFFFu; }
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_if(uint32_t bar, uint32_t bytes, uint32_t lead) {
+    asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes), "r"(lead) : "memory");
+}
+// One lane of the warp, the same one every time.  The warps that drive the copy engine and the tensor cores run their loops with all lanes
+// and let `lead` predicate the single-thread instructions: inside a branch that one lane takes, the operands of those instructions live
+// in per-thread registers and every issue pays for moving them to uniform ones (measured: 80 clocks a tcgen05.mma, 630 a k-step of any
+// width; without the branch the k-step runs at the tensor rate).
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t lead;
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(lead));
+    return lead;
+}
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint32_t lead) {   // arrives at the barrier of that offset in both CTAs
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"((uint16_t)3), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t (&a)[32], uint32_t taddr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, "
+        "%25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]), "=r"(a[8]), "=r"(a[9]), "=r"(a[10]), "=r"(a[11]),
+          "=r"(a[12]), "=r"(a[13]), "=r"(a[14]), "=r"(a[15]), "=r"(a[16]), "=r"(a[17]), "=r"(a[18]), "=r"(a[19]), "=r"(a[20]), "=r"(a[21]), "=r"(a[22]), "=r"(a[23]),
+          "=r"(a[24]), "=r"(a[25]), "=r"(a[26]), "=r"(a[27]), "=r"(a[28]), "=r"(a[29]), "=r"(a[30]), "=r"(a[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -140,138 +208,196 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;                             // SWIZZLE_128B
     return d;
 }
-__host__ __device__ constexpr uint32_t umma_idesc_i8(int a_signed, int b_signed, int bn = kGemmBN) {
-    return (2u << 4)                        // D format S32
-           | ((uint32_t)a_signed << 7)      // A: 0 unsigned / 1 signed 8-bit
-           | ((uint32_t)b_signed << 10)     // B
-           | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kGemmBM >> 4) << 24);   // K-major A and B (bits 15, 16 = 0)
+// One tile of the pair kernel: 256 weight columns (128 a CTA) x T tokens, T a multiple of 32 up to 160 chosen by i8_tile_tokens()
+struct PairGemmArgs {
+    GemmArgs g;
+    int T;             // tokens of a tile
+    int tiles_t, tiles;
+    int* err;          // set to 1 when a wait ran out
+};
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+        "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void tc_mma_i8_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
+        : "memory");
+}
+__host__ __device__ constexpr uint32_t umma_idesc_i8_mn(int a_signed, int b_signed, int m, int n) {
+    return (2u << 4) | ((uint32_t)a_signed << 7) | ((uint32_t)b_signed << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);   // D format S32
+}
+// the integer sum of a (column, token) as fp32: exact in 64 bits, then one rounding (the GEMV epilogue's expression)
+__device__ __forceinline__ float digits_to_float(int a2, int a1, int a0, long long off) {
+    const long long t = ((long long)a2 << 16) + ((long long)a1 << 8) + (long long)a0 - off;
+    const int hi = (int)(t >> 23), lo = (int)(t & 0x7FFFFF);
+    return fmaf((float)hi, 8388608.0f, (float)lo);
+}
+// tokens of a tile: waves of the pairs times what they cost in clocks -- a k-step takes 6 a token at the tensor rate or its bytes at
+// 60 a clock, a tile its epilogue on top (the accumulators of a wide tile fill TMEM, so the next tile starts behind it)
+inline int i8_tile_tokens(int M, int n_tiles, int ksteps, int pairs) {
+    int best = 160;
+    float best_t = 1e30f;
+    for (int T = 160; T >= 32; T -= 32) {
+        const int waves = (((M + T - 1) / T) * n_tiles + pairs - 1) / pairs;
+        const float step = std::max(6.f * T, (kGemmTileBytes + 192.f * T) / 60.f);
+        const float t = waves * (ksteps * step + 1500.f + 20.f * T);
+        if (t < best_t) { best_t = t; best = T; }
+    }
+    return best;
 }
 
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const GemmArgs g) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const PairGemmArgs pg) {
     extern __shared__ uint8_t gsm_raw[];
+    const GemmArgs& g = pg.g;
     const uint32_t base = (smem_u32(gsm_raw) + 1023u) & ~1023u;
     uint8_t* tiles = gsm_raw + (base - smem_u32(gsm_raw));
     uint64_t* full = reinterpret_cast<uint64_t*>(tiles + (size_t)kGemmStages * kGemmStageBytes);
     uint64_t* empty = full + kGemmStages;
-    uint64_t* tmem_full = empty + kGemmStages;
-    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_full + 1);
+    uint64_t* acc_full = empty + kGemmStages;
+    uint64_t* acc_empty = acc_full + 1;       // the even CTA's: both CTAs' epilogue warps
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 1);
+    float* s_sx = reinterpret_cast<float*>(tiles + (size_t)kGemmStages * kGemmStageBytes + 256);        // [160] of the tile's tokens
+    long long* s_sxf = reinterpret_cast<long long*>(s_sx + kGemmMaxTokens);                            // [160]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nb = blockIdx.x, mb = blockIdx.y;
-    const int KB = g.k_pad / kGemmBK;
+    const uint32_t rank = cluster_ctarank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int KB = g.k_pad / kGemmBK, T = pg.T;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kGemmStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        mbar_init(tmem_full, 1);
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, 2 * kGemmEpiWarps);
         fence_mbar_init();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_ptr)) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_ptr)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    pdl_wait_prior_grid();   // (everything above touches only this CTA: it runs under the tail of the kernel before)
     tc_fence_before();
     __syncthreads();
+    cluster_sync_all();      // the peer's barriers are initialised before anything is signalled across
     tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
 
     if (warp == 0) {
-        if (lane == 0) {
+        const uint32_t lead = elect_one();
+        const uint32_t bytes = 2u * (uint32_t)(kGemmTileBytes + 3 * (T / 2) * kGemmBK);   // both CTAs' boxes (rows beyond the tensors arrive as zeros and count)
+        const uint32_t full_s = smem_u32(full);
+        bool ok = true;
+        int st = 0, use = 0;
+        for (int tile = pair; tile < pg.tiles && ok; tile += pairs) {
+            const int tb = tile % pg.tiles_t, nb = tile / pg.tiles_t;
+            const int tok = tb * T + (int)rank * (T / 2), wrow = (2 * nb + (int)rank) * KB * kGemmBN;
             for (int kb = 0; kb < KB; ++kb) {
-                const int st = kb % kGemmStages, use = kb / kGemmStages;
-                if (use > 0) mbar_wait(&empty[st], (use - 1) & 1);
-                mbar_arrive_expect_tx(&full[st], kGemmStageBytes);
-                uint8_t* sbase = tiles + (size_t)st * kGemmStageBytes;
-                for (int d = 0; d < 3; ++d) tma_load_2d(sbase + d * kGemmTileBytes, &map_a, kb * kGemmBK, d * g.m_pad + mb * kGemmBM, &full[st]);
-                bulk_g2s(sbase + 3 * kGemmTileBytes, g.wt + ((size_t)nb * KB + kb) * kGemmTileBytes, kGemmTileBytes, &full[st]);
+                if (use > 0 && !(ok = mbar_wait_bounded(&empty[st], (use - 1) & 1, pg.err))) break;
+                const uint32_t sbase = base + st * kGemmStageBytes, bar = pair_leader(full_s + 8 * st);
+                if (rank == 0) mbar_expect_tx_if(full_s + 8 * st, bytes, lead);
+                tma_load_2d_pair(sbase, &map_w, 0, wrow + kb * kGemmBN, bar, lead);
+                tma_load_3d_pair(sbase + kGemmTileBytes, &map_x, kb * kGemmBK, tok, 0, bar, lead);
+                if (++st == kGemmStages) { st = 0; ++use; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t id_s = umma_idesc_i8(1, g.a_signed_b);   // A = signed digit plane
-            for (int kb = 0; kb < KB; ++kb) {
-                const int st = kb % kGemmStages, use = kb / kGemmStages;
-                mbar_wait(&full[st], use & 1);
+        if (rank == 0) {
+            const uint32_t lead = elect_one();
+            const uint32_t idesc = umma_idesc_i8_mn(g.a_signed_b, 1, 256, T);   // A = weights (unsigned nibbles in bytes or signed bytes), B = signed digits
+            const uint64_t desc0 = umma_desc_sw128(base);   // (addresses stay below 2^18: adding to the address field never carries out of it)
+            const uint32_t empty_s = smem_u32(empty), plane = (uint32_t)(T / 2) * kGemmBK >> 4;
+            bool ok = true;
+            int st = 0, use = 0, n_tile = 0;
+            for (int tile = pair; tile < pg.tiles && ok; tile += pairs, ++n_tile) {
+                if (n_tile > 0) ok = mbar_wait_bounded(acc_empty, (n_tile - 1) & 1, pg.err);
                 tc_fence_after();
-                const uint32_t sbase = base + st * kGemmStageBytes;
+                for (int kb = 0; kb < KB && ok; ++kb) {
+                    ok = mbar_wait_bounded(&full[st], use & 1, pg.err);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t wd = desc0 + (uint64_t)(st * (kGemmStageBytes >> 4)), xd = wd + (kGemmTileBytes >> 4);
 #pragma unroll
-                for (int k4 = 0; k4 < kGemmBK / 32; ++k4) {
-                    const uint64_t bdesc = umma_desc_sw128(sbase + 3 * kGemmTileBytes + k4 * 32);
+                    for (int k4 = 0; k4 < kGemmBK / 32; ++k4)
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        const uint64_t adesc = umma_desc_sw128(sbase + d * kGemmTileBytes + k4 * 32);
-                        tc_mma_i8(tmem + d * kGemmBN, adesc, bdesc, id_s, (kb | k4) != 0 ? 1u : 0u);
-                    }
+                        for (int d = 0; d < 3; ++d)
+                            tc_mma_i8_pair(tmem + d * T, wd + 2 * k4, xd + d * plane + 2 * k4, idesc, (kb | k4) != 0 ? 1u : 0u, lead);
+                    tc_commit_pair(empty_s + 8 * st, lead);
+                    if (++st == kGemmStages) { st = 0; ++use; }
                 }
-                tc_commit(&empty[st]);   // the stage may be refilled once these MMAs have read it
+                tc_commit_pair(smem_u32(acc_full), lead);   // also on the failure path: the epilogue warps must not wait for ever
             }
-            tc_commit(tmem_full);
         }
     } else {
-        // epilogue: warp w may touch TMEM lanes 32*(w%4) .. +31; lane = token row of the tile
-        mbar_wait(tmem_full, 0);
-        tc_fence_after();
-        const int q = warp & 3;
-        const int row = mb * kGemmBM + q * 32 + lane;
-        const bool row_ok = row < g.M;
-        const float sx = row_ok ? g.sx[row] : 0.f;
-        const long long sxf = row_ok ? g.sxf[row] : 0;
-        const long long offterm = (long long)g.woff * sxf;
-        const float fsxf = (float)sxf;
-        for (int c0 = 0; c0 < kGemmBN; c0 += 16) {
-            uint32_t a[3][16];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(d * kGemmBN + c0);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                    : "=r"(a[d][0]), "=r"(a[d][1]), "=r"(a[d][2]), "=r"(a[d][3]), "=r"(a[d][4]), "=r"(a[d][5]), "=r"(a[d][6]), "=r"(a[d][7]),
-                      "=r"(a[d][8]), "=r"(a[d][9]), "=r"(a[d][10]), "=r"(a[d][11]), "=r"(a[d][12]), "=r"(a[d][13]), "=r"(a[d][14]), "=r"(a[d][15])
-                    : "r"(taddr));
+        // TMEM lane = weight column, TMEM column = token: a store of a warp is 32 neighbouring columns of one token
+        const int q = warp & 3, half = (warp - 2) >> 2, et = threadIdx.x - 64;
+        bool ok = true;
+        int n_tile = 0;
+        // (after a failed wait the loop goes on without waiting or storing: the warps meet at the same barriers to the end)
+        for (int tile = pair; tile < pg.tiles; tile += pairs, ++n_tile) {
+            const int tb = tile % pg.tiles_t, nb = tile / pg.tiles_t;
+            const int tok0 = tb * T;
+            bar_sync(1, 32 * kGemmEpiWarps);   // the previous tile's token numbers are no longer read
+            if (et < T) {
+                const bool in = tok0 + et < g.M;
+                s_sx[et] = in ? g.sx[tok0 + et] : 0.f;
+                s_sxf[et] = in ? g.sxf[tok0 + et] : 0;
             }
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row_ok) {
-                auto val = [&](int i, int n) -> float {
-                    const long long t = ((long long)(int)a[2][i] << 16) + ((long long)(int)a[1][i] << 8) + (long long)(int)a[0][i] - offterm;
-                    const int hi = (int)(t >> 23), lo = (int)(t & 0x7FFFFF);
-                    const float tf = fmaf((float)hi, 8388608.0f, (float)lo);
-                    const float zt = g.colzterm ? g.colzterm[n] : 0.f;
-                    return (fmaf(zt, fsxf, tf) * sx) * g.colscale[n];   // the GEMV epilogue's expression
-                };
-                const int nbase = nb * kGemmBN + c0;
-                float* yrow = g.y + (size_t)row * g.N;
-                const float* rrow = g.resid ? g.resid + (size_t)row * g.N : nullptr;
-                if ((g.N & 3) == 0 && nbase + 16 <= g.N) {   // 64 contiguous bytes per lane: four 16-byte stores
+            bar_sync(1, 32 * kGemmEpiWarps);
+            const int n = (2 * nb + (int)rank) * kGemmBN + q * 32 + lane;
+            const bool n_ok = n < g.N;
+            const float cs = n_ok ? g.colscale[n] : 0.f;
+            const float zt = (n_ok && g.colzterm) ? g.colzterm[n] : 0.f;
+            if (ok) ok = mbar_wait_bounded(acc_full, n_tile & 1, pg.err);
+            ok = __all_sync(0xffffffffu, ok);
+            tc_fence_after();
+            const int c1 = min((half + 1) * (T / 2), g.M - tok0);
+            for (int c0 = half * (T / 2); ok && c0 < c1; c0 += 16) {
+                uint32_t a[3][16];
 #pragma unroll
-                    for (int i = 0; i < 16; i += 4) {
-                        float4 v = make_float4(val(i, nbase + i), val(i + 1, nbase + i + 1), val(i + 2, nbase + i + 2), val(i + 3, nbase + i + 3));
-                        if (rrow) {
-                            const float4 r = *reinterpret_cast<const float4*>(rrow + nbase + i);
-                            v.x = r.x + v.x; v.y = r.y + v.y; v.z = r.z + v.z; v.w = r.w + v.w;
-                        }
-                        *reinterpret_cast<float4*>(yrow + nbase + i) = v;
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int n = nbase + i;
-                        if (n < g.N) {
-                            float yv = val(i, n);
-                            if (rrow) yv = rrow[n] + yv;
-                            yrow[n] = yv;
-                        }
-                    }
+                for (int d = 0; d < 3; ++d) {
+                    const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(d * T + c0);
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                        : "=r"(a[d][0]), "=r"(a[d][1]), "=r"(a[d][2]), "=r"(a[d][3]), "=r"(a[d][4]), "=r"(a[d][5]), "=r"(a[d][6]), "=r"(a[d][7]),
+                          "=r"(a[d][8]), "=r"(a[d][9]), "=r"(a[d][10]), "=r"(a[d][11]), "=r"(a[d][12]), "=r"(a[d][13]), "=r"(a[d][14]), "=r"(a[d][15])
+                        : "r"(taddr));
                 }
+                float r[16];
+                const size_t at = (size_t)(tok0 + c0) * g.N + n;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) r[i] = (g.resid && n_ok && c0 + i < c1) ? g.resid[at + (size_t)i * g.N] : 0.f;
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const long long sxf = s_sxf[c0 + i];
+                    const float tf = digits_to_float((int)a[2][i], (int)a[1][i], (int)a[0][i], g.woff * sxf);
+                    v[i] = ((g.colzterm ? fmaf(zt, (float)sxf, tf) : tf) * s_sx[c0 + i]) * cs;
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (n_ok && c0 + i < c1) g.y[at + (size_t)i * g.N] = g.resid ? r[i] + v[i] : v[i];
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(pair_leader(smem_u32(acc_empty)));
         }
-        tc_fence_before();
     }
+    tc_fence_before();
     __syncthreads();
+    cluster_sync_all();   // nothing of the peer's is in flight towards this CTA's shared memory or TMEM any more
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }
 }
-
 
 // ---- the same GEMM for M <= 32 rows (batched decode), operands swapped ---------------------------------------------
 // With a handful of rows the kernel above would spend 128-row MMAs and 48 KiB of (mostly zero) activation tiles on 32 live
@@ -315,10 +441,6 @@ struct SplitKArgs {
     int n_pad;
     long long* dbg;           // optional (microbenchmark): SM-clock stamps of CTA (0, 0)
 };
-
-__host__ __device__ constexpr uint32_t umma_idesc_i8_mn(int a_signed, int b_signed, int m, int n) {
-    return (2u << 4) | ((uint32_t)a_signed << 7) | ((uint32_t)b_signed << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
 
 __global__ void __launch_bounds__(kSmallThreads, 1)
 gemm_i8_tc_small_kernel(const GemmArgs g, const SplitKArgs sk) {

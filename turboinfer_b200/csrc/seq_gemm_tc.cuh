@@ -43,17 +43,6 @@ struct TcArgs {
     int* err;   // set to 1 when a wait ran out
 };
 
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* err) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (clock64() - t0 > 2000000000LL) {   // about a second
-            atomicExch(err, 1);
-            return false;
-        }
-    }
-    return true;
-}
 // D fp32, A and B bf16, both K-major
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
@@ -79,44 +68,6 @@ inline int pair_tile_columns(int M, int N, int K, int pairs) {
     return best;
 }
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// the shared-memory address of the even CTA's copy of a barrier (bit 24 of a shared::cluster address is the CTA's place in its pair)
-__device__ __forceinline__ uint32_t pair_leader(uint32_t saddr) { return saddr & 0xFEFFFFFFu; }
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar, uint32_t lead) {
-    asm volatile(
-        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %5, 0;\n\t"
-        "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar), "r"(lead)
-        : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx_if(uint32_t bar, uint32_t bytes, uint32_t lead) {
-    asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes), "r"(lead) : "memory");
-}
-// One lane of the warp, the same one every time.  The warps that drive the copy engine and the tensor cores run their loops with all lanes
-// and let `lead` predicate the single-thread instructions: inside a branch that one lane takes, the operands of those instructions live
-// in per-thread registers and every issue pays for moving them to uniform ones (measured: 80 clocks a tcgen05.mma, 630 a k-step of any
-// width; without the branch the k-step runs at the tensor rate).
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t lead;
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(lead));
-    return lead;
-}
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint32_t lead) {   // arrives at the barrier of that offset in both CTAs
-    asm volatile(
-        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
-        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"((uint16_t)3), "r"(lead)
-        : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t lead) {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\t"
@@ -126,17 +77,6 @@ __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t tmem_d, uint64_t adesc
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t (&a)[32], uint32_t taddr) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, "
-        "%25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]), "=r"(a[8]), "=r"(a[9]), "=r"(a[10]), "=r"(a[11]),
-          "=r"(a[12]), "=r"(a[13]), "=r"(a[14]), "=r"(a[15]), "=r"(a[16]), "=r"(a[17]), "=r"(a[18]), "=r"(a[19]), "=r"(a[20]), "=r"(a[21]), "=r"(a[22]), "=r"(a[23]),
-          "=r"(a[24]), "=r"(a[25]), "=r"(a[26]), "=r"(a[27]), "=r"(a[28]), "=r"(a[29]), "=r"(a[30]), "=r"(a[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 // four neighbouring results of one row to where they belong: C through the epilogue, or the activated columns
 __device__ __forceinline__ void pair_put4(const TcArgs& g, int row, int n, float4 v) {
     const GluCols& u = g.cols;
