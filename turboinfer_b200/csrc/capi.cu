@@ -168,8 +168,8 @@ int set_kernel_attrs() {
     CK(cudaFuncSetAttribute(causal_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPfSmemBytes));
     CK(cudaFuncSetAttribute(causal_attention_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_tc_smem_bytes<128>()));
     CK(cudaFuncSetAttribute(causal_attention_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_tc_smem_bytes<64>()));
-    CK(cudaFuncSetAttribute(causal_attention_h3_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_h3_smem_bytes<128>()));
-    CK(cudaFuncSetAttribute(causal_attention_h3_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_h3_smem_bytes<64>()));
+    CK(cudaFuncSetAttribute(attn_tc_kernel<128, 128, PrefillAttn>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_tc_smem_bytes5<128, 128>()));
+    CK(cudaFuncSetAttribute(attn_tc_kernel<64, 64, PrefillAttn>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_tc_smem_bytes5<64, 64>()));
     CK(cudaFuncSetAttribute(sample_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 176 * 1024));
     CK(cudaFuncSetAttribute(sample_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 176 * 1024));
     CK(cudaFuncSetAttribute(beam_expand_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 176 * 1024));
@@ -390,6 +390,7 @@ struct Model {
     int pf_cap = 0;
     float last_prefill_ms = 0.f;   // CUDA-event time of the prompt phase of the last generate call
     DevBuf<float> pf_x, pf_qkv, pf_attn, pf_gu, pf_act, pf_sx;
+    DevBuf<uint8_t> pf_images;   // split keys and values of the prefill attention
     DevBuf<int8_t> pf_planes;
     DevBuf<long long> pf_sxf;
     DevBuf<unsigned long long> pf_ws;   // split-K workspace of the 32-row GEMM: [n_pad][32] integer partial sums, zero between GEMMs
@@ -1254,6 +1255,29 @@ bool prefill_gemm_eligible(const Model& m, int M) {
     return true;
 }
 
+// causal attention of M prompt rows at positions pos0 .. on tcgen05: the heads' keys and values are split into tile images, as many heads
+// at a time as the image buffer takes (a buffer that cannot be had is asked for in halves, down to one head)
+template <int DH>
+int prefill_attention(Model& m, Layer& ly, int M, int pos0, float scale) {
+    const int H = m.cfg.hidden, heads = m.attn_heads, n = pos0 + M, kt = (n + kAtKT - 1) / kAtKT;
+    int per = at_heads_per_launch(heads, kt, DH, DH, kAtImageBudget);
+    while (m.pf_images.n < (size_t)per * kt * at_record_bytes(DH, DH)) {
+        if (m.pf_images.alloc((size_t)per * kt * at_record_bytes(DH, DH)) == 0) break;
+        cudaGetLastError();
+        if (per == 1) return 1;
+        per = (per + 1) / 2;
+    }
+    for (int h0 = 0; h0 < heads; h0 += per) {
+        const int nh = std::min(per, heads - h0);
+        const PrefillKeys keys{ly.k_pool.p, ly.v_pool.p, m.page_table.p, m.page_tokens, H, DH, DH, n, h0};
+        const PrefillAttn shape{m.pf_qkv.p, m.pf_attn.p, M, H, DH, DH, 1, h0, pos0, scale};
+        kv_images_kernel<DH, DH, PrefillKeys><<<dim3(kt, nh), 256, 0, g_stream>>>(keys, m.pf_images.p);
+        attn_tc_kernel<DH, DH, PrefillAttn><<<dim3(nh, (M + kAtQ - 1) / kAtQ), kAtThreads, attn_tc_smem_bytes5<DH, DH>(), g_stream>>>(shape, m.pf_images.p, g_gemm_err_dev);
+        g_launches += h0 == 0 ? 1 : 2;   // (the caller counts one)
+    }
+    return 0;
+}
+
 // forward_pass over prompt[0 .. M): fills the KV cache for positions pos0 .. pos0 + M - 1 (pos0 = 0 after reset()).
 // The hidden states stay in pf_x; the caller runs the last prompt token through the decode engine for the logits.
 int ensure_pf_scratch(Model& m, int M);
@@ -1273,13 +1297,10 @@ int prefill_gemm(Model& m, const int* prompt_dev, int M) {
         static const std::string attn_sel = getenv("TURBOINFER_B200_PREFILL_ATTN") ? getenv("TURBOINFER_B200_PREFILL_ATTN") : "";   // A/B: fp32 | tf32
         const bool attn_fp32 = attn_sel == "fp32", attn_tf32 = attn_sel == "tf32";
         const float att_scale = 1.0f / sqrtf((float)m.attn_dim);
-        const dim3 tc_grid(m.attn_heads, (M + kTcQ - 1) / kTcQ);
-        if (!attn_fp32 && !attn_tf32 && m.attn_dim == 128) {          // tensor cores, split FP16 (prefill.cuh)
-            causal_attention_h3_kernel<128><<<tc_grid, kTcThreads, attn_h3_smem_bytes<128>(), g_stream>>>(
-                m.pf_qkv.p, M, H, att_scale, pos0, ly.k_pool.p, ly.v_pool.p, m.page_table.p, m.page_tokens, m.pf_attn.p);
+        if (!attn_fp32 && !attn_tf32 && m.attn_dim == 128) {          // tcgen05, split FP16 (attn_tc.cuh)
+            TRY(prefill_attention<128>(m, ly, M, pos0, att_scale));
         } else if (!attn_fp32 && !attn_tf32 && m.attn_dim == 64) {
-            causal_attention_h3_kernel<64><<<tc_grid, kTcThreads, attn_h3_smem_bytes<64>(), g_stream>>>(
-                m.pf_qkv.p, M, H, att_scale, pos0, ly.k_pool.p, ly.v_pool.p, m.page_table.p, m.page_tokens, m.pf_attn.p);
+            TRY(prefill_attention<64>(m, ly, M, pos0, att_scale));
         } else if (!attn_fp32 && m.attn_dim == 128) {   // split TF32
             causal_attention_tc_kernel<128><<<dim3(m.attn_heads, (M + kTcQ - 1) / kTcQ), kTcThreads, attn_tc_smem_bytes<128>(), g_stream>>>(
                 m.pf_qkv.p, M, H, att_scale, pos0, ly.k_pool.p, ly.v_pool.p, m.page_table.p, m.page_tokens, m.pf_attn.p);

@@ -8,7 +8,7 @@
 // All fp32, full-precision expf / division like the decode path.
 #pragma once
 #include <cuda_fp16.h>
-#include "gemm_tc.cuh"
+#include "attn_tc.cuh"
 
 namespace tib {
 
@@ -405,14 +405,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) causal_attention_tc_kernel(cons
 }
 
 // ---------------------------------------------------------------------------------------------------
-// The same attention with FP16 MMAs (mma.sync m16n8k16, twice the work per instruction of the TF32 form): every fp32 operand
-// is split into two halves, x = hi + lo (hi = fp16(x), lo = fp16(x - hi): 22 mantissa bits), and hi*hi + hi*lo + lo*hi is
-// accumulated in fp32 -- the accuracy of the split-TF32 kernel above at half its instruction count.  Values are activations
-// (|x| well inside fp16's range).  Q, K, V hi / lo images live in shared memory as halves ([row][D + 8]: conflict-free
-// ldmatrix / LDS.32); K fragments come from ldmatrix, V fragments from ldmatrix.trans (the k index of P V is the key), and the
-// C fragments of two adjacent S tiles ARE the A fragment of P V for 16 keys, so P never leaves registers.
+// Warp-level FP16 MMAs on operands split into two halves, x = hi + lo (hi = fp16(x), lo = fp16(x - hi): 22 mantissa bits), hi*hi + hi*lo +
+// lo*hi accumulated in fp32: the pieces the latent and the head-mixing attention of the sequence engine are made of.
 // ---------------------------------------------------------------------------------------------------
-template <int DH> constexpr size_t attn_h3_smem_bytes() { return ((size_t)2 * kTcQ + 4 * kTcKT) * (DH + 8) * sizeof(__half); }
 __device__ __forceinline__ void split_h(float x, __half& hi, __half& lo) {
     hi = __float2half_rn(x);
     lo = __float2half_rn(x - __half2float(hi));
@@ -431,154 +426,42 @@ __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t saddr) {
 __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t saddr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr));
 }
-template <int DH>
-__global__ void __launch_bounds__(kTcThreads, 1) causal_attention_h3_kernel(const float* qkv, int M, int H, float scale, int pos0, const float* k_pool,
-                                                                              const float* v_pool, const int* page_table, int page_tokens, float* out) {
-    constexpr int LD = DH + 8, KS = DH / 16, NT = DH / 8;   // row stride in halves; k-steps of Q K^T; n-tiles of P V
-    extern __shared__ __align__(16) __half h3_smem[];
-    __half* Qh = h3_smem;                 // [128][LD]
-    __half* Ql = Qh + kTcQ * LD;
-    __half* Kh = Ql + kTcQ * LD;          // [64][LD]
-    __half* Kl = Kh + kTcKT * LD;
-    __half* Vh = Kl + kTcKT * LD;
-    __half* Vl = Vh + kTcKT * LD;
-    const int h = blockIdx.x, qb = (int)(gridDim.y - 1 - blockIdx.y) * kTcQ;   // latest queries (most key tiles) first
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int hoff = h * DH;
-    const int r0 = qb + 16 * warp + g, r1 = r0 + 8;
-    auto store_split4 = [](const float4& v, __half* hi, __half* lo) {
-        __half a[4], b[4];
-        split_h(v.x, a[0], b[0]); split_h(v.y, a[1], b[1]); split_h(v.z, a[2], b[2]); split_h(v.w, a[3], b[3]);
-        *reinterpret_cast<uint2*>(hi) = make_uint2(pack_h2(a[0], a[1]), pack_h2(a[2], a[3]));
-        *reinterpret_cast<uint2*>(lo) = make_uint2(pack_h2(b[0], b[1]), pack_h2(b[2], b[3]));
-    };
-    for (int i = tid; i < kTcQ * (DH / 4); i += kTcThreads) {
-        const int q = i / (DH / 4), d4 = (i % (DH / 4)) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (qb + q < M) v = *reinterpret_cast<const float4*>(qkv + (size_t)(qb + q) * 3 * H + hoff + d4);
-        store_split4(v, Qh + q * LD + d4, Ql + q * LD + d4);
+// ---- the default attention of the prefill, head dimensions 64 and 128: attn_tc.cuh over the paged cache (which already holds the rows' own K / V)
+struct PrefillKeys {   // kv_images_kernel: key t of the prompt
+    const float *k_pool, *v_pool;
+    const int* page_table;
+    int page_tokens, H, d, dv, n, g0;
+    struct Tile { int t0; };
+    __device__ bool tile(int x, Tile& t) const { t.t0 = x * kAtKT; return true; }
+    __device__ const float* row(const Tile& tile, int r, int g, bool is_v) const {
+        const int t = tile.t0 + r;
+        if (t >= n) return nullptr;
+        return (is_v ? v_pool : k_pool) + ((size_t)page_table[t / page_tokens] * page_tokens + t % page_tokens) * H + (size_t)g * d;
     }
-    float o[NT][4];
-#pragma unroll
-    for (int n = 0; n < NT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-    const int last_pos = pos0 + min(qb + kTcQ, M) - 1;
-    const int warp_last = pos0 + min(qb + 16 * warp + 15, M - 1);
-    // A fragments of Q: rows g / g + 8 of the warp's 16, halves (2t, 2t + 1) and (2t + 8, 2t + 9) of a 16-dim k-step
-    const uint32_t* qh_row = reinterpret_cast<const uint32_t*>(Qh + (16 * warp + g) * LD) + t;
-    const uint32_t* ql_row = reinterpret_cast<const uint32_t*>(Ql + (16 * warp + g) * LD) + t;
-    // ldmatrix row addresses: lane -> (matrix = lane / 8, row = lane % 8)
-    const int lm = lane >> 3, lr = lane & 7;
-    const uint32_t k_ld = (uint32_t)(((lr + 8 * (lm >> 1)) * LD + 8 * (lm & 1)) * 2);   // K: matrices (keys 0-7 | dims 0-7, 8-15), (keys 8-15 | ...)
-    const uint32_t v_ld = (uint32_t)(((lr + 8 * (lm & 1)) * LD + 8 * (lm >> 1)) * 2);   // V^T: matrices (keys 0-7, 8-15 | dims 0-7), (... | dims 8-15)
-    const uint32_t kh_s = smem_u32(Kh), kl_s = smem_u32(Kl), vh_s = smem_u32(Vh), vl_s = smem_u32(Vl);
-    for (int t0 = 0; t0 <= last_pos; t0 += kTcKT) {
-        __syncthreads();
-        for (int i = tid; i < kTcKT * (DH / 4); i += kTcThreads) {
-            const int kk = i / (DH / 4), d4 = (i % (DH / 4)) * 4, tk = t0 + kk;
-            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-            if (tk <= last_pos) {
-                const size_t row = ((size_t)page_table[tk / page_tokens] * page_tokens + (tk % page_tokens)) * H + hoff + d4;
-                kv = *reinterpret_cast<const float4*>(k_pool + row);
-                vv = *reinterpret_cast<const float4*>(v_pool + row);
-            }
-            store_split4(kv, Kh + kk * LD + d4, Kl + kk * LD + d4);
-            store_split4(vv, Vh + kk * LD + d4, Vl + kk * LD + d4);
-        }
-        __syncthreads();
-        if (t0 > warp_last) continue;
-        // ---- S = Q K^T ----
-        float sc[kTcKT / 8][4];
-#pragma unroll
-        for (int j = 0; j < kTcKT / 8; ++j) sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < KS; ++ks) {
-            const uint32_t ah[4] = {qh_row[8 * ks], qh_row[8 * ks + 4 * LD], qh_row[8 * ks + 4], qh_row[8 * ks + 4 * LD + 4]};   // (LD halves = LD / 2 words; 8 rows = 4 LD words)
-            const uint32_t al[4] = {ql_row[8 * ks], ql_row[8 * ks + 4 * LD], ql_row[8 * ks + 4], ql_row[8 * ks + 4 * LD + 4]};
-#pragma unroll
-            for (int jp = 0; jp < kTcKT / 16; ++jp) {   // two key tiles per ldmatrix.x4: {b0, b1} of tile 2 jp, {b0, b1} of tile 2 jp + 1
-                uint32_t bh[4], bl[4];
-                const uint32_t off = (uint32_t)((16 * jp * LD + 16 * ks) * 2) + k_ld;
-                ldsm_x4(bh, kh_s + off);
-                ldsm_x4(bl, kl_s + off);
-                mma_f16(sc[2 * jp], al, bh[0], bh[1]);
-                mma_f16(sc[2 * jp + 1], al, bh[2], bh[3]);
-                mma_f16(sc[2 * jp], ah, bl[0], bl[1]);
-                mma_f16(sc[2 * jp + 1], ah, bl[2], bl[3]);
-                mma_f16(sc[2 * jp], ah, bh[0], bh[1]);
-                mma_f16(sc[2 * jp + 1], ah, bh[2], bh[3]);
-            }
-        }
-        // ---- online softmax (as in the TF32 kernel) ----
-        const int qp0 = pos0 + r0, qp1 = pos0 + r1;
-        float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < kTcKT / 8; ++j) {
-            const int key = t0 + 8 * j + 2 * t;
-            sc[j][0] = (key <= qp0 && r0 < M) ? sc[j][0] * scale : -INFINITY;
-            sc[j][1] = (key + 1 <= qp0 && r0 < M) ? sc[j][1] * scale : -INFINITY;
-            sc[j][2] = (key <= qp1 && r1 < M) ? sc[j][2] * scale : -INFINITY;
-            sc[j][3] = (key + 1 <= qp1 && r1 < M) ? sc[j][3] * scale : -INFINITY;
-            mx0 = fmaxf(mx0, fmaxf(sc[j][0], sc[j][1]));
-            mx1 = fmaxf(mx1, fmaxf(sc[j][2], sc[j][3]));
-        }
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-        float rs0 = 0.f, rs1 = 0.f;
-#pragma unroll
-        for (int j = 0; j < kTcKT / 8; ++j) {
-            sc[j][0] = mn0 == -INFINITY ? 0.f : expf(sc[j][0] - mn0);
-            sc[j][1] = mn0 == -INFINITY ? 0.f : expf(sc[j][1] - mn0);
-            sc[j][2] = mn1 == -INFINITY ? 0.f : expf(sc[j][2] - mn1);
-            sc[j][3] = mn1 == -INFINITY ? 0.f : expf(sc[j][3] - mn1);
-            rs0 += sc[j][0] + sc[j][1];
-            rs1 += sc[j][2] + sc[j][3];
-        }
-        rs0 += __shfl_xor_sync(0xffffffffu, rs0, 1); rs0 += __shfl_xor_sync(0xffffffffu, rs0, 2);
-        rs1 += __shfl_xor_sync(0xffffffffu, rs1, 1); rs1 += __shfl_xor_sync(0xffffffffu, rs1, 2);
-        const float c0 = mn0 == -INFINITY ? 1.f : expf(m0 - mn0), c1 = mn1 == -INFINITY ? 1.f : expf(m1 - mn1);
-        l0 = l0 * c0 + rs0;
-        l1 = l1 * c1 + rs1;
-        m0 = mn0;
-        m1 = mn1;
-#pragma unroll
-        for (int n = 0; n < NT; ++n) { o[n][0] *= c0; o[n][1] *= c0; o[n][2] *= c1; o[n][3] *= c1; }
-        // ---- O += P V: k-step jp = keys 16 jp .. 16 jp + 15 = S tiles 2 jp and 2 jp + 1 ----
-#pragma unroll
-        for (int jp = 0; jp < kTcKT / 16; ++jp) {
-            uint32_t ph[4], pl[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {   // a0: (row g, keys 2t, 2t+1) a1: (row g+8, ...) of tile 2 jp; a2, a3: the same of tile 2 jp + 1
-                const float x = sc[2 * jp + (i >> 1)][2 * (i & 1)], y = sc[2 * jp + (i >> 1)][2 * (i & 1) + 1];
-                __half xh, xl, yh, yl;
-                split_h(x, xh, xl);
-                split_h(y, yh, yl);
-                ph[i] = pack_h2(xh, yh);
-                pl[i] = pack_h2(xl, yl);
-            }
-#pragma unroll
-            for (int np = 0; np < NT / 2; ++np) {   // two dim tiles per ldmatrix.x4.trans
-                uint32_t bh[4], bl[4];
-                const uint32_t off = (uint32_t)((16 * jp * LD + 16 * np) * 2) + v_ld;
-                ldsm_x4_trans(bh, vh_s + off);
-                ldsm_x4_trans(bl, vl_s + off);
-                mma_f16(o[2 * np], pl, bh[0], bh[1]);
-                mma_f16(o[2 * np + 1], pl, bh[2], bh[3]);
-                mma_f16(o[2 * np], ph, bl[0], bl[1]);
-                mma_f16(o[2 * np + 1], ph, bl[2], bl[3]);
-                mma_f16(o[2 * np], ph, bh[0], bh[1]);
-                mma_f16(o[2 * np + 1], ph, bh[2], bh[3]);
-            }
-        }
+};
+struct PrefillAttn {
+    const float* qkv;
+    float* out;
+    int M, H, d, dv, group, h0, pos0;
+    float scale;
+    __device__ void tile(int y, int& row0, int& count, int& p0, int& image0) const {
+        row0 = (int)(gridDim.y - 1 - y) * kAtQ;   // latest queries (most key tiles) first: no long tail
+        count = min(kAtQ, M - row0);
+        p0 = pos0 + row0;
+        image0 = 0;
     }
-    const float i0 = 1.0f / l0, i1 = 1.0f / l1;
+    __device__ const float* q(int row, int h) const { return qkv + (size_t)row * 3 * H + (size_t)h * d; }
+    __device__ int first_key(int) const { return 0; }
+    __device__ void scores(float (&s)[kAtKT]) const {
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        if (r0 < M) *reinterpret_cast<float2*>(out + (size_t)r0 * H + hoff + 8 * n + 2 * t) = make_float2(o[n][0] * i0, o[n][1] * i0);
-        if (r1 < M) *reinterpret_cast<float2*>(out + (size_t)r1 * H + hoff + 8 * n + 2 * t) = make_float2(o[n][2] * i1, o[n][3] * i1);
+        for (int j = 0; j < kAtKT; ++j) s[j] *= scale;
     }
-}
+    __device__ bool sigmoid() const { return false; }
+    __device__ float pb(int) const { return 0.f; }
+    __device__ float sigmoid_weight(float, float) const { return 0.f; }
+    __device__ float finish(int, int, float, float l) const { return 1.0f / l; }
+    __device__ void store4(int row, int h, int c, float4 v) const { *reinterpret_cast<float4*>(out + (size_t)row * H + (size_t)h * d + c) = v; }
+};
 
 // act[m][i] = up * silu(gate) from interleaved columns (gate_i, up_i) of gu[M][2I]
 __global__ void swiglu_rows_kernel(const float* gu, float* act, size_t M, size_t I) {

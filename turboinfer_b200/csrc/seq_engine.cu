@@ -266,6 +266,7 @@ struct Model {
     int max_aux = 0, max_aux2 = 0, max_route = 0;
     bool any_rgbuf = false;
     DevBuf<int> meta, picks;
+    DevBuf<uint8_t> kv_images;   // split keys and values of the portions' attention (one layer run's, rewritten by the next)
     DevBuf<__nv_bfloat16> abf;   // bf16 copy of a product's activations for the tcgen05 path: [rows][max_k]
     DevBuf<int> attn_arrived;    // split-key attention: finished splits of a (row, head), zero between launches
     DevBuf<float> attn_part;     // split-key attention partials: [rows][heads][splits][vdim + 2]
@@ -1048,9 +1049,20 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
             r0 += counts[e];
         }
     }
+    // the split key tiles of the portions' attention: every page of a portion's sequence, entry by entry
+    std::vector<int> ktiles, image0;
+    if (!tiles128.empty() && m.d.mode == TI_SEQ_BF16) {
+        image0.assign(E, 0);
+        for (int e = 0; e < E; ++e) {
+            if (counts[e] < kAttnTiledMinRows) continue;
+            image0[e] = (int)ktiles.size() / 2;
+            for (int p = 0; p < (m.seqs[seqs[e]].len + counts[e] + kPageTokens - 1) / kPageTokens; ++p) { ktiles.push_back(e); ktiles.push_back(p); }
+        }
+    }
+    const int n_ktiles = (int)ktiles.size() / 2;
     const size_t n_xtable = xpages.empty() ? 0 : (size_t)m.seqs.size() * stride;
     const size_t n_meta = (size_t)3 * T + (size_t)(E + 1) + 2 * (size_t)E + (size_t)std::max(n_out, 1) + (size_t)m.seqs.size() * stride +
-                          (size_t)3 * T + 4 + mtiles.size() + row_tile.size() + xpages.size() + n_xtable;
+                          (size_t)3 * T + 4 + mtiles.size() + row_tile.size() + xpages.size() + n_xtable + ktiles.size() + image0.size();
     if (n_meta > m.meta_host_cap) {
         if (m.meta_host) cudaFreeHost(m.meta_host);
         m.meta_host = nullptr;
@@ -1100,6 +1112,9 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
         for (int e = 0; e < E; ++e)
             for (int p = 0; xfirst[e] >= 0 && p < (int)m.seqs[seqs[e]].pages.size(); ++p) h_xtable[(size_t)seqs[e] * stride + p] = xfirst[e] + p;
     }
+    int* h_ktiles = h_xtable + n_xtable;
+    std::copy(ktiles.begin(), ktiles.end(), h_ktiles);
+    std::copy(image0.begin(), image0.end(), h_ktiles + ktiles.size());
     // the previous step's copy out of this pinned buffer has completed: every step ends with a stream synchronisation
     CK(cudaMemcpyAsync(m.meta.p, hp, n_meta * sizeof(int), cudaMemcpyHostToDevice, g_stream));
     StepMeta sm{};
@@ -1118,6 +1133,8 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     const int* d_row_tile = d_mtiles + mtiles.size();
     const int* d_xpages = d_row_tile + row_tile.size();
     const int* d_xtable = d_xpages + xpages.size();
+    const int* d_ktiles = d_xtable + n_xtable;
+    const int* d_image0 = d_ktiles + ktiles.size();
     sm.table_stride = stride;
     sm.T = T;
     sm.E = E;
@@ -1227,16 +1244,33 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     // paged softmax attention of all rows of the step (prompt portions in tiles, the other rows one by one or split over their keys)
     auto h3_size = [](const AttnShape& s) { return s.dim <= 128 && s.vdim <= 128 && s.dim % 4 == 0 && s.vdim % 4 == 0 && s.v_ld == 0; };
     auto h3_attention = [&](const StepMeta& sm, const AttnShape& s, const float* q, const float* kp, const float* vp, float* out) -> int {   // the portions' tiles
-        const dim3 grid(s.heads, n_tiles128);
-        const int dk = s.dim <= 64 ? 64 : 128, dv = s.vdim <= 64 ? 64 : 128;
-        const bool sized = dk == s.dim && dv == s.vdim;
-#define TI_H3_CASE(K, V, X) window_attention_h3_kernel<K, V, X><<<grid, kTcThreads, window_h3_smem_bytes<K, V>(), g_stream>>>(q, sm, s, d_tiles128, kp, vp, out)
-        if (dk == 64 && dv == 64) { if (sized) TI_H3_CASE(64, 64, true); else TI_H3_CASE(64, 64, false); }
-        else if (dk == 128 && dv == 128) { if (sized) TI_H3_CASE(128, 128, true); else TI_H3_CASE(128, 128, false); }
-        else if (dk == 64) TI_H3_CASE(64, 128, false);
-        else TI_H3_CASE(128, 64, false);
-#undef TI_H3_CASE
-        LAUNCHED();
+        const int dk = at_pad(s.dim), dv = at_pad(s.vdim), group = s.heads / s.kv_heads;
+        // keys and values are split into tile images first, as many heads at a time as the image buffer takes (a buffer that cannot be had
+        // is asked for in halves, down to one head)
+        int per = at_heads_per_launch(s.kv_heads, n_ktiles, dk, dv, kAtImageBudget);
+        while (m.kv_images.n < (size_t)per * n_ktiles * at_record_bytes(dk, dv)) {
+            if (m.kv_images.alloc((size_t)per * n_ktiles * at_record_bytes(dk, dv)) == 0) break;
+            cudaGetLastError();
+            if (per == 1) return 1;
+            per = (per + 1) / 2;
+        }
+        for (int g0 = 0; g0 < s.kv_heads; g0 += per) {
+            const int ng = std::min(per, s.kv_heads - g0);
+            const SeqKeys keys{sm, s, d_ktiles, kp, vp, s.dim, s.vdim, g0};
+            const SeqAttn shape{sm, s, d_tiles128, d_image0, q, out, s.dim, s.vdim, group, g0 * group};
+#define TI_AT_CASE(K, V)                                                                                                                               \
+    {                                                                                                                                                  \
+        kv_images_kernel<K, V, SeqKeys><<<dim3(n_ktiles, ng), 256, 0, g_stream>>>(keys, m.kv_images.p);                                                \
+        attn_tc_kernel<K, V, SeqAttn><<<dim3(ng * group, n_tiles128), kAtThreads, attn_tc_smem_bytes5<K, V>(), g_stream>>>(shape, m.kv_images.p, m.err.p); \
+    }
+            if (dk == 64 && dv == 64) TI_AT_CASE(64, 64)
+            else if (dk == 128 && dv == 128) TI_AT_CASE(128, 128)
+            else if (dk == 64) TI_AT_CASE(64, 128)
+            else TI_AT_CASE(128, 64)
+#undef TI_AT_CASE
+            LAUNCHED();
+            LAUNCHED();
+        }
         return 0;
     };
     auto attention = [&](const AttnShape& s, const float* q, const float* kp, const float* vp, float* out, bool only_small = false) -> int {   // (only_small: not the portions)
@@ -2064,14 +2098,12 @@ int ti_seq_init(int device) {
     if (const char* e = getenv("TURBOINFER_B200_SEQ_PDL")) g_use_pdl = atoi(e) != 0;
     if (const char* e = getenv("TURBOINFER_B200_SEQ_ROW_MMA")) g_use_row_mma = atoi(e) != 0;
     if (const char* e = getenv("TURBOINFER_B200_SEQ_TILED_ATTN")) g_use_tiled_attn = atoi(e) != 0;
-#define TI_H3_ATTR(K, V, X) CK(cudaFuncSetAttribute(window_attention_h3_kernel<K, V, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)window_h3_smem_bytes<K, V>()))
-    TI_H3_ATTR(64, 64, true);
-    TI_H3_ATTR(64, 64, false);
-    TI_H3_ATTR(128, 128, true);
-    TI_H3_ATTR(128, 128, false);
-    TI_H3_ATTR(64, 128, false);
-    TI_H3_ATTR(128, 64, false);
-#undef TI_H3_ATTR
+#define TI_AT_ATTR(K, V) CK(cudaFuncSetAttribute(attn_tc_kernel<K, V, SeqAttn>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_tc_smem_bytes5<K, V>()))
+    TI_AT_ATTR(64, 64);
+    TI_AT_ATTR(128, 128);
+    TI_AT_ATTR(64, 128);
+    TI_AT_ATTR(128, 64);
+#undef TI_AT_ATTR
     CK(cudaFuncSetAttribute(window_attention_tiled_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_smem_optin));
     CK(cudaFuncSetAttribute(window_attention_tiled_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_smem_optin));
     CK(cudaFuncSetAttribute(window_attention_tiled_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_smem_optin));
