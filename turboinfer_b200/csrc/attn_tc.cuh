@@ -86,20 +86,6 @@ __device__ __forceinline__ void tc_mma_f16_if(uint32_t tmem_d, uint64_t adesc, u
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
-__device__ __forceinline__ void tc_commit_if(uint32_t bar, uint32_t lead) {
-    asm volatile(
-        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead)
-        : "memory");
-}
-__device__ __forceinline__ void bulk_g2s_if(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint32_t lead) {
-    asm volatile(
-        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %4, 0;\n\t"
-        "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(dst),
-        "l"(src), "r"(bytes), "r"(bar), "r"(lead)
-        : "memory");
-}
-
 // Shape: tile(y, row0, count, pos0, image0) -- the rows of the block, the position of the first, the record of the sequence's key tile 0;
 // d, dv (multiples of four), h0 (first query head of the launch), group (query heads a key/value head); q(row, h); first_key(pos), never
 // later for an earlier row; scores(): scales (and caps) raw products; sigmoid(): weights sigmoid_weight(score, pb(h)) instead of a softmax;

@@ -35,7 +35,7 @@ constexpr int kGemmStages = 4, kGemmEpiWarps = 8;
 constexpr int kGemmThreads = 64 + 32 * kGemmEpiWarps;
 constexpr int kGemmTileBytes = kGemmBN * kGemmBK;              // 16 KiB of weights
 constexpr int kGemmStageBytes = kGemmTileBytes + 3 * (kGemmMaxTokens / 2) * kGemmBK;   // + three digit planes of half the tile's tokens: 46 KiB
-constexpr size_t kGemmSmemBytes = (size_t)kGemmStages * kGemmStageBytes + 1024 /*align*/ + 256 /*barriers*/ + kGemmMaxTokens * 12 /*s_x, sum(xf)*/;
+constexpr size_t kGemmSmemBytes = (size_t)kGemmStages * kGemmStageBytes + 1024 /*align*/ + 256 /*barriers*/ + kGemmMaxTokens * 16 /*the tokens' numbers*/;
 
 struct GemmArgs {
     int M, N, K;            // logical sizes
@@ -120,16 +120,8 @@ __global__ void unpack_kmajor_kernel(const uint8_t* packed, QLayout L, int k_pad
 }
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(smem_dst)),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-                 : "memory");
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* err) {
     if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
@@ -190,12 +182,27 @@ __device__ __forceinline__ void tmem_ld32(uint32_t (&a)[32], uint32_t taddr) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_commit_if(uint32_t bar, uint32_t lead) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void bulk_g2s_if(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %4, 0;\n\t"
+        "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(dst),
+        "l"(src), "r"(bytes), "r"(bar), "r"(lead)
+        : "memory");
+}
+
+__device__ __forceinline__ void tc_mma_i8_if(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
 // K-major, SWIZZLE_128B, tile rows 128 B apart inside 1024-byte 8-row groups
@@ -234,9 +241,9 @@ __device__ __forceinline__ void tc_mma_i8_pair(uint32_t tmem_d, uint64_t adesc, 
 __host__ __device__ constexpr uint32_t umma_idesc_i8_mn(int a_signed, int b_signed, int m, int n) {
     return (2u << 4) | ((uint32_t)a_signed << 7) | ((uint32_t)b_signed << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);   // D format S32
 }
-// the integer sum of a (column, token) as fp32: exact in 64 bits, then one rounding (the GEMV epilogue's expression)
-__device__ __forceinline__ float digits_to_float(int a2, int a1, int a0, long long off) {
-    const long long t = ((long long)a2 << 16) + ((long long)a1 << 8) + (long long)a0 - off;
+// the integer sum of a (column, token), and it as fp32: exact in 64 bits, then one rounding (the GEMV epilogue's expression)
+__device__ __forceinline__ long long digits_sum(int a2, int a1, int a0) { return ((long long)a2 << 16) + ((long long)a1 << 8) + (long long)a0; }
+__device__ __forceinline__ float int_to_float(long long t) {
     const int hi = (int)(t >> 23), lo = (int)(t & 0x7FFFFF);
     return fmaf((float)hi, 8388608.0f, (float)lo);
 }
@@ -265,8 +272,9 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     uint64_t* acc_full = empty + kGemmStages;
     uint64_t* acc_empty = acc_full + 1;       // the even CTA's: both CTAs' epilogue warps
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 1);
-    float* s_sx = reinterpret_cast<float*>(tiles + (size_t)kGemmStages * kGemmStageBytes + 256);        // [160] of the tile's tokens
-    long long* s_sxf = reinterpret_cast<long long*>(s_sx + kGemmMaxTokens);                            // [160]
+    // [160] of the tile's tokens: woff * sum(xf), then {s_x, sum(xf)}
+    long long* s_off = reinterpret_cast<long long*>(tiles + (size_t)kGemmStages * kGemmStageBytes + 256);
+    float2* s_x = reinterpret_cast<float2*>(s_off + kGemmMaxTokens);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -346,8 +354,9 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             bar_sync(1, 32 * kGemmEpiWarps);   // the previous tile's token numbers are no longer read
             if (et < T) {
                 const bool in = tok0 + et < g.M;
-                s_sx[et] = in ? g.sx[tok0 + et] : 0.f;
-                s_sxf[et] = in ? g.sxf[tok0 + et] : 0;
+                const long long sxf = in ? g.sxf[tok0 + et] : 0;
+                s_off[et] = g.woff * sxf;
+                s_x[et] = make_float2(in ? g.sx[tok0 + et] : 0.f, (float)sxf);
             }
             bar_sync(1, 32 * kGemmEpiWarps);
             const int n = (2 * nb + (int)rank) * kGemmBN + q * 32 + lane;
@@ -377,9 +386,9 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 float v[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const long long sxf = s_sxf[c0 + i];
-                    const float tf = digits_to_float((int)a[2][i], (int)a[1][i], (int)a[0][i], g.woff * sxf);
-                    v[i] = ((g.colzterm ? fmaf(zt, (float)sxf, tf) : tf) * s_sx[c0 + i]) * cs;
+                    const float2 x = s_x[c0 + i];
+                    const float tf = int_to_float(digits_sum((int)a[2][i], (int)a[1][i], (int)a[0][i]) - s_off[c0 + i]);
+                    v[i] = (fmaf(zt, x.y, tf) * x.x) * cs;   // (zt = 0 without a zero point: the sum itself)
                 }
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
@@ -399,239 +408,233 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
 }
 
-// ---- the same GEMM for M <= 32 rows (batched decode), operands swapped ---------------------------------------------
-// With a handful of rows the kernel above would spend 128-row MMAs and 48 KiB of (mostly zero) activation tiles on 32 live
-// rows.  Here the roles are swapped: the MMA's M side (128 rows) are 128 WEIGHT COLUMNS, its N side (32) are the batch
-// rows, D[128 x 32] per digit plane (96 TMEM columns):
-//   * per k-step a CTA loads 16 KiB of weights and the 32 live rows of each digit plane (12 KiB -- the same bytes for
-//     every CTA, an L2 broadcast), both stored as ready-made swizzled tile images and fetched with 1-D bulk copies;
-//   * the tensor work is 4x smaller than with padded rows, and the epilogue has all four warps busy with coalesced stores
-//     (lane = weight column);
-//   * 7 stages of 28 KiB: what bounds a CTA is the chain of TMA round trips of its k-loop (measured: with 3 stages a
-//     32-step loop took 21 us whatever else the chip was doing), so the ring is as deep as shared memory allows;
-//   * split-K: grid (N / 128, S); CTA (n, s) multiplies k-steps [s KB / S, (s + 1) KB / S).  The partial sums are exact
-//     integers, so they are combined with 64-bit integer atomics in a workspace (order-independent: bit-identical to
-//     S = 1); the CTA that arrives last on the tile's counter applies offset, scales and residual, stores the tile and
-//     leaves workspace and counter zeroed for the next GEMM.  S is chosen on the host for GEMMs with few column tiles.
-// warps 0..3: epilogue (TMEM lanes 32w.. = weight columns), warp 4: TMEM allocation + MMA issue, warp 5: TMA producer.
-#ifndef TIB_SMALL_TILES
-#define TIB_SMALL_TILES 1
-#endif
-// A pipeline stage holds kSmallTiles consecutive k-tiles (each: weights 16 KiB + digits 12 KiB, fetched as ready-made images).
-// Stages of two or three k-tiles (fewer mbarrier polls per byte at the same ~170-196 KiB in flight) were measured and are no
-// faster (7B, batch 32: 5.34 ms per step with 1 tile x 7 stages, 5.37 with 2 x 3, 5.48 with 3 x 2): the polls are not what paces
-// the k-loop.  Kept as a compile-time knob.
-constexpr int kSmallTiles = TIB_SMALL_TILES;
-constexpr int kSmallRows = 32, kSmallThreads = 192, kSmallStages = kSmallTiles == 1 ? 7 : (kSmallTiles == 2 ? 3 : 2);
-constexpr int kSmallPlaneBytes = kSmallRows * kGemmBK;                       // 4 KiB
-constexpr int kSmallTileBytes = kGemmTileBytes + 3 * kSmallPlaneBytes;       // one k-tile: weights 16 KiB + digits 12 KiB
-constexpr int kSmallStageBytes = kSmallTiles * kSmallTileBytes;
-constexpr int kSmallTmemCols = 512;                                          // four accumulator sets of 3 x 32 columns
-constexpr size_t kSmallSmemBytes = (size_t)kSmallStages * kSmallStageBytes + 1024 /*align*/ + 256 /*barriers*/ + 2 * kSmallRows * 8;
+// ---- the same GEMM for M <= 32 rows (batched decode), operands swapped, dealt evenly to the SMs ------------------------
+// With a handful of rows the work is a stream of weights.  The MMA's M side (128 rows) are 128 WEIGHT COLUMNS, its N side R batch rows
+// (16 or 32) of all three digit planes at once, D[128 x 3 R].  The (column tile, k-step) units of the whole matrix are numbered tile by
+// tile and every CTA takes one contiguous run of them, so that all SMs stream the same number of bytes whatever the number of
+// column tiles (172 tiles of a 4096 x 22016 matrix on 148 SMs would otherwise be two waves); a run covers the end of a tile, whole tiles, the
+// beginning of another.
+//   * per k-step a CTA loads 16 KiB of weights and 3 R digit rows (6 or 12 KiB -- the same bytes for every CTA, an L2 broadcast), both stored
+//     as ready-made swizzled tile images and fetched with 1-D bulk copies into a ring of 196 KiB; under programmatic dependent launch
+//     the first ring of WEIGHTS is requested while the kernel before (which makes the digits) still runs;
+//   * a tile that several CTAs share: each leaves its partial sums (exact integers) in its own place of a workspace and counts itself in;
+//     the CTA that arrives last adds them (order-independent: bit-identical to an unshared tile), applies offset, scales and residual, and
+//     leaves the counter zeroed for the next GEMM;
+//   * two accumulators: the epilogue of a tile runs under the k-steps of the next.
+// warps 0..7: epilogue (warp w: weight columns 32 (w % 4) .., rows 16 (w / 4) ..), warp 8: TMEM allocation + MMA issue, warp 9: producer.
+// Measured (INT4 weights, 32 rows, us a launch in a chain of launches on a B200; before: whole column tiles, K split into at most eight):
+// see small_gemm_ctas() for the rule.
+constexpr int kSmallRows = 32, kSmallEpiWarps = 8, kSmallThreads = 64 + 32 * kSmallEpiWarps;
+constexpr int kSmallRing = 196 * 1024;
+constexpr int kSmallTmemCols = 256;                                          // two accumulators of up to 96 columns
+constexpr size_t kSmallSmemBytes = (size_t)kSmallRing + 1024 /*align*/ + 256 /*barriers*/ + kSmallRows * 16 /*the rows' numbers*/;
+__host__ __device__ constexpr int small_stage_bytes(int R) { return kGemmTileBytes + 3 * R * kGemmBK; }   // 28 KiB (7 stages) or 22 KiB (8 of 9)
+__host__ __device__ constexpr int small_stages(int R) { return R == 32 ? 7 : 8; }
+// the digit planes of a step's rows are laid out for 16 or for 32 rows
+TIB_HD int small_rows(int M) { return M <= 16 ? 16 : 32; }
 
-// The digit planes of the 32 rows for this kernel: [k-step][96 rows = 32 d + m][128 B], each k-step's 12 KiB the exact
-// SWIZZLE_128B image of the three plane tiles (one bulk copy per k-step)
-TIB_HD size_t xtile_offset(int d, int m, int k) {
-    return (size_t)(k / kGemmBK) * 3 * 4096 + sw128_offset(d * 32 + m, k % kGemmBK);
+// The digit planes for this kernel: [k-step][3 R rows = R d + m][128 B], each k-step's rows the exact SWIZZLE_128B image (one bulk copy)
+TIB_HD size_t xtile_offset(int d, int m, int k, int R) {
+    return (size_t)(k / kGemmBK) * 3 * R * kGemmBK + sw128_offset(d * R + m, k % kGemmBK);
 }
-struct SplitKArgs {
+struct SmallArgs {
     const uint8_t* xt;        // digit planes in xtile_offset order
-    unsigned long long* ws;   // [32][n_pad] partial integer sums
-    unsigned int* cnt;        // [N / 128] arrivals per tile
-    int n_pad;
-    long long* dbg;           // optional (microbenchmark): SM-clock stamps of CTA (0, 0)
+    long long* ws;            // [2 CTAs][32][128] partial sums: a CTA's first and last tile when they are shared
+    unsigned int* cnt;        // [column tiles] arrivals, zero between GEMMs
+    int tiles, KB;            // column tiles, k-steps
+    int* err;                 // set to 1 when a wait ran out
 };
+// first unit of CTA c (units * CTAs fits 32 bits: at most 2^22 units on 148 SMs)
+TIB_HD int small_unit(int units, int c, int ctas) { return (int)((uint32_t)units * (uint32_t)c / (uint32_t)ctas); }
+// CTAs of a launch: all SMs as long as each has at least `min_steps` k-steps (below that the fix-up of shared tiles costs more than it gives)
+inline int small_gemm_ctas(int units, int sms) { return std::max(1, std::min(sms, units / 4)); }
 
+template <int R>
 __global__ void __launch_bounds__(kSmallThreads, 1)
-gemm_i8_tc_small_kernel(const GemmArgs g, const SplitKArgs sk) {
+gemm_i8_tc_small_kernel(const GemmArgs g, const SmallArgs sk) {
+    constexpr int kStages = small_stages(R), kStageBytes = small_stage_bytes(R), kCols = 3 * R;
+    static_assert(kStages * kStageBytes <= kSmallRing, "ring");
     extern __shared__ uint8_t gsm_raw[];
     const uint32_t base = (smem_u32(gsm_raw) + 1023u) & ~1023u;
     uint8_t* tiles = gsm_raw + (base - smem_u32(gsm_raw));
-    uint64_t* full = reinterpret_cast<uint64_t*>(tiles + (size_t)kSmallStages * kSmallStageBytes);
-    uint64_t* empty = full + kSmallStages;
-    uint64_t* tmem_full = empty + kSmallStages;
-    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_full + 1);
+    uint64_t* full = reinterpret_cast<uint64_t*>(tiles + kSmallRing);
+    uint64_t* empty = full + kStages;
+    uint64_t* acc_full = empty + kStages;     // [2]
+    uint64_t* acc_empty = acc_full + 2;       // [2]
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* flag = reinterpret_cast<int*>(tmem_ptr + 1);
-    float* s_sx = reinterpret_cast<float*>(tiles + (size_t)kSmallStages * kSmallStageBytes + 256);
-    long long* s_off = reinterpret_cast<long long*>(s_sx + kSmallRows);   // woff * sum(xf) per row; sum(xf) itself after it
+    long long* s_off = reinterpret_cast<long long*>(tiles + kSmallRing + 256);   // [32]: woff * sum(xf) per row, then {s_x, sum(xf)}
+    float2* s_x = reinterpret_cast<float2*>(s_off + kSmallRows);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nb = blockIdx.x, S = gridDim.y;
-    const int KB = g.k_pad / kGemmBK;
-    const int kb0 = (int)((long long)blockIdx.y * KB / S), kb1 = (int)((long long)(blockIdx.y + 1) * KB / S);
-    // Every CTA reads the SAME digit-plane tiles; marching through k in lockstep would make all of them hit the same L2
-    // lines at the same moment (measured: ~1.2 us per k-step whatever the pipeline depth).  Each column tile therefore
-    // starts its k-loop at a different offset and wraps around -- integer sums do not care about the order.
-    const int nk = kb1 - kb0, rot = nk > 0 ? (int)((blockIdx.x * 7u) % (unsigned)nk) : 0;
-    const int ns = (nk + kSmallTiles - 1) / kSmallTiles;   // pipeline stages of this CTA: stage i = k-tiles [i * kSmallTiles, ...) of its (rotated) range
+    const int KB = sk.KB, units = sk.tiles * KB, ctas = gridDim.x;
+    const int u0 = small_unit(units, blockIdx.x, ctas), u1 = small_unit(units, blockIdx.x + 1, ctas);
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kSmallStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        mbar_init(tmem_full, 1);
+        for (int i = 0; i < kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kSmallEpiWarps); }
         fence_mbar_init();
     }
-    if (warp == 4) {
+    if (warp == 8) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr)), "n"(kSmallTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    // Everything above touches shared memory and TMEM only: under programmatic dependent launch (the lockstep step's graph) it
-    // overlaps the tail of the previous kernel; the activations, scales and split-K workspace are read after this point.
-    pdl_wait_prior_grid();
-    pdl_launch_dependents();
-    if (threadIdx.x < kSmallRows) {
-        const bool ok = (int)threadIdx.x < g.M;
-        s_sx[threadIdx.x] = ok ? g.sx[threadIdx.x] : 0.f;
-        s_off[threadIdx.x] = ok ? g.sxf[threadIdx.x] : 0;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
+    pdl_launch_dependents();
 
-    // Both pipeline loops poll mbarriers, and a poll costs ~0.1-0.2 us even when the phase is long complete (measured,
-    // scripts/microbench7.cu) -- as much as a whole 28 KiB k-step should take.  So four lanes probe the next four stages
-    // at once (lane 0 blocking, the others non-blocking) and lane 0 then handles every consecutive stage that is ready.
-    auto probe4 = [&](uint64_t* bars, int i, int phase_flip) -> int {
-        const int j = i + lane;
-        bool ok = false;
-        if (lane < 4 && j < ns) {
-            const int stj = j % kSmallStages;
-            const uint32_t parj = (uint32_t)((j / kSmallStages) & 1) ^ (uint32_t)phase_flip;
-            ok = lane == 0 ? mbar_try_wait(&bars[stj], parj) : mbar_test_wait(&bars[stj], parj);
-        }
-        const unsigned int mask = __ballot_sync(0xffffffffu, ok) & 0xFu;
-        return __ffs(~mask) - 1;   // consecutive ready stages from i on (0..4)
-    };
-    if (warp == 5) {
-        int i = 0;
-        while (i < ns) {
-            const int nready = probe4(empty, i, 1);   // a fresh mbarrier counts its "previous" phase as complete
-            if (lane == 0) {
-                for (int q = 0; q < nready; ++q) {
-                    const int ii = i + q, st = ii % kSmallStages;
-                    const int ntile = min(kSmallTiles, nk - ii * kSmallTiles);
-                    if (sk.dbg && blockIdx.x == 0 && blockIdx.y == 0 && ii < 40) sk.dbg[64 + ii] = clock64();
-                    mbar_arrive_expect_tx(&full[st], (uint32_t)(ntile * kSmallTileBytes));
-                    for (int j = 0; j < ntile; ++j) {
-                        const int tt = ii * kSmallTiles + j;
-                        const int kb = kb0 + (tt + rot < nk ? tt + rot : tt + rot - nk);
-                        uint8_t* sbase = tiles + (size_t)st * kSmallStageBytes + (size_t)j * kSmallTileBytes;
-                        bulk_g2s(sbase, g.wt + ((size_t)nb * KB + kb) * kGemmTileBytes, kGemmTileBytes, &full[st]);
-                        bulk_g2s(sbase + kGemmTileBytes, sk.xt + (size_t)kb * 3 * kSmallPlaneBytes, 3 * kSmallPlaneBytes, &full[st]);
-                    }
-                }
-            }
-            __syncwarp();
-            i += nready;
-        }
-    } else if (warp == 4) {
-        // A = weights (unsigned nibbles-in-bytes for INT4, signed for INT8); B = ALL THREE signed digit planes at once:
-        // their 32-row tiles are contiguous in the stage, so one MMA with N = 96 fills the three accumulators
-        // (columns 32 d + m) of the k4 step's accumulator set.
-        const uint32_t id = umma_idesc_i8_mn(g.a_signed_b, 1, kGemmBN, 3 * kSmallRows);
-        int i = 0;
-        while (i < ns) {
-            const int nready = probe4(full, i, 0);
-            if (lane == 0 && nready > 0) {
-                tc_fence_after();
-                for (int q = 0; q < nready; ++q) {
-                    const int ii = i + q, st = ii % kSmallStages;
-                    const int ntile = min(kSmallTiles, nk - ii * kSmallTiles);
-                    if (sk.dbg && blockIdx.x == 0 && blockIdx.y == 0 && ii < 40) sk.dbg[128 + ii] = clock64();
-                    for (int j = 0; j < ntile; ++j) {
-                        const uint32_t sbase = base + st * kSmallStageBytes + j * kSmallTileBytes;
-#pragma unroll
-                        for (int k4 = 0; k4 < kGemmBK / 32; ++k4) {
-                            const uint64_t wdesc = umma_desc_sw128(sbase + k4 * 32);
-                            const uint64_t xdesc = umma_desc_sw128(sbase + kGemmTileBytes + k4 * 32);
-                            // one accumulator set per k4: four independent accumulation chains; the epilogue adds the sets
-                            tc_mma_i8(tmem + k4 * 3 * kSmallRows, wdesc, xdesc, id, (ii | j) != 0 ? 1u : 0u);
-                        }
-                    }
-                    tc_commit(&empty[st]);   // the stage may be refilled once these MMAs have read it
-                }
-            }
-            __syncwarp();
-            i += nready;
-        }
-        if (lane == 0) tc_commit(tmem_full);
-    } else {
-        // epilogue, warps 0..3: TMEM lane = weight column of the tile, TMEM column = batch row (per digit plane)
-        if (sk.dbg && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) sk.dbg[0] = clock64();
-        mbar_wait(tmem_full, 0);
-        tc_fence_after();
-        if (sk.dbg && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) sk.dbg[1] = clock64();
-        const int n = nb * kGemmBN + warp * 32 + lane;
-        const bool n_ok = n < g.N;
-        const float cs = n_ok ? g.colscale[n] : 0.f;
-        const float zt = (n_ok && g.colzterm) ? g.colzterm[n] : 0.f;
-        auto finish = [&](int m, long long t) {   // t = sum over all k of u * xf for (row m, column n)
-            const long long sxf = s_off[m];
-            t -= (long long)g.woff * sxf;
-            const int hi = (int)(t >> 23), lo = (int)(t & 0x7FFFFF);
-            const float tf = fmaf((float)hi, 8388608.0f, (float)lo);
-            float yv = (fmaf(zt, (float)sxf, tf) * s_sx[m]) * cs;   // the GEMV epilogue's expression
-            if (g.resid) yv = g.resid[(size_t)m * g.N + n] + yv;
-            g.y[(size_t)m * g.N + n] = yv;
+    if (warp == 9) {
+        const uint32_t lead = elect_one();
+        const uint32_t full_s = smem_u32(full);
+        auto weights = [&](int u, int st) {
+            mbar_expect_tx_if(full_s + 8 * st, (uint32_t)kStageBytes, lead);
+            bulk_g2s_if(base + st * kStageBytes, g.wt + (size_t)u * kGemmTileBytes, kGemmTileBytes, full_s + 8 * st, lead);   // (units are in the images' order)
         };
-        for (int m0 = 0; m0 < kSmallRows; m0 += 16) {
-            uint32_t a[3][16];
+        auto digits = [&](int u, int st) {
+            bulk_g2s_if(base + st * kStageBytes + kGemmTileBytes, sk.xt + (size_t)(u % KB) * kCols * kGemmBK, kCols * kGemmBK, full_s + 8 * st, lead);
+        };
+        const int ahead = min(kStages, u1 - u0);
+        for (int i = 0; i < ahead; ++i) weights(u0 + i, i);
+        pdl_wait_prior_grid();
+        for (int i = 0; i < ahead; ++i) digits(u0 + i, i);
+        bool ok = true;
+        for (int u = u0 + ahead, st = 0, use = 1; u < u1 && ok; ++u) {
+            ok = mbar_wait_bounded(&empty[st], (use - 1) & 1, sk.err);
+            weights(u, st);
+            digits(u, st);
+            if (++st == kStages) { st = 0; ++use; }
+        }
+    } else if (warp == 8) {
+        // A = weights (unsigned nibbles-in-bytes for INT4, signed for INT8); B = all three signed digit planes at once: their rows are
+        // contiguous in the stage, so one MMA with N = 3 R fills the three accumulators (columns R d + m)
+        const uint32_t lead = elect_one();
+        const uint32_t id = umma_idesc_i8_mn(g.a_signed_b, 1, kGemmBN, kCols);
+        const uint64_t desc0 = umma_desc_sw128(base);
+        const uint32_t empty_s = smem_u32(empty);
+        bool ok = true;
+        int st = 0, use = 0, n_seg = 0;
+        for (int u = u0; u < u1 && ok; ++n_seg) {
+            const int buf = n_seg & 1, end = min(u1, (u / KB + 1) * KB), begin = u;
+            if (n_seg > 1) ok = mbar_wait_bounded(&acc_empty[buf], ((n_seg >> 1) - 1) & 1, sk.err);
+            tc_fence_after();
+            for (; u < end && ok; ++u) {
+                ok = mbar_wait_bounded(&full[st], use & 1, sk.err);
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t wd = desc0 + (uint64_t)(st * (kStageBytes >> 4)), xd = wd + (kGemmTileBytes >> 4);
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
+                for (int k4 = 0; k4 < kGemmBK / 32; ++k4) tc_mma_i8_if(tmem + buf * 128, wd + 2 * k4, xd + 2 * k4, id, (u != begin || k4 != 0) ? 1u : 0u, lead);
+                tc_commit_if(empty_s + 8 * st, lead);
+                if (++st == kStages) { st = 0; ++use; }
+            }
+            tc_commit_if(smem_u32(&acc_full[buf]), lead);   // also on the failure path: the epilogue warps must not wait for ever
+        }
+    } else {
+        // epilogue: TMEM lane = weight column of the tile, TMEM column = batch row (per digit plane)
+        pdl_wait_prior_grid();
+        if (threadIdx.x < R) {
+            const bool in = (int)threadIdx.x < g.M;
+            const long long sxf = in ? g.sxf[threadIdx.x] : 0;
+            s_off[threadIdx.x] = g.woff * sxf;
+            s_x[threadIdx.x] = make_float2(in ? g.sx[threadIdx.x] : 0.f, (float)sxf);
+        }
+        bar_sync(1, 32 * kSmallEpiWarps);
+        bool ok = true;
+        int n_seg = 0;
+        const int tile0 = u0 / KB, q = warp & 3, col = q * 32 + lane, m0 = 16 * (warp >> 2);
+        const bool active = m0 < g.M;
+        // (after a failed wait the loop goes on without storing: the warps meet at the same barriers to the end)
+        for (int u = u0; u < u1; ++n_seg) {
+            const int buf = n_seg & 1, tile = u / KB, end = min(u1, (tile + 1) * KB);
+            const bool whole = u == tile * KB && end == (tile + 1) * KB;
+            u = end;
+            const int n = tile * kGemmBN + col;
+            const bool n_ok = n < g.N;
+            const float cs = n_ok ? g.colscale[n] : 0.f;
+            const float zt = (n_ok && g.colzterm) ? g.colzterm[n] : 0.f;
+            // a shared tile: the CTAs c0 .. c1 whose runs touch it
+            int c0 = 0, c1 = 0;
+            if (!whole) {
+                const int first = tile * KB, last = first + KB - 1;
+                c0 = (int)((uint32_t)first * (uint32_t)ctas / (uint32_t)units);
+                while (small_unit(units, c0 + 1, ctas) <= first) ++c0;
+                c1 = (int)((uint32_t)last * (uint32_t)ctas / (uint32_t)units);
+                while (c1 + 1 < ctas && small_unit(units, c1 + 1, ctas) <= last) ++c1;
+            }
+            if (ok) ok = mbar_wait_bounded(&acc_full[buf], (n_seg >> 1) & 1, sk.err);
+            ok = __all_sync(0xffffffffu, ok);
+            tc_fence_after();
+            auto finish = [&](const long long (&t)[16]) {   // t[i] = sum over all k of u * xf for (row m0 + i, column n)
+                float r[16], y[16];
+                const size_t at = (size_t)m0 * g.N + n;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) a[d][i] = 0u;
+                for (int i = 0; i < 16; ++i) r[i] = (g.resid && n_ok && m0 + i < g.M) ? g.resid[at + (size_t)i * g.N] : 0.f;
 #pragma unroll
-                for (int set = 0; set < kGemmBK / 32; ++set) {
-                    uint32_t b[16];
-                    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(set * 3 * kSmallRows + d * kSmallRows + m0);
+                for (int i = 0; i < 16; ++i) {
+                    const float2 x = s_x[m0 + i];
+                    y[i] = (fmaf(zt, x.y, int_to_float(t[i] - s_off[m0 + i])) * x.x) * cs;   // the GEMV epilogue's expression
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (n_ok && m0 + i < g.M) g.y[at + (size_t)i * g.N] = g.resid ? r[i] + y[i] : y[i];
+            };
+            constexpr int kPlace = kSmallRows * kGemmBN;
+            if (active && ok) {
+                uint32_t a[3][16];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 128 + d * R + m0);
                     asm volatile(
                         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                        : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7]),
-                          "=r"(b[8]), "=r"(b[9]), "=r"(b[10]), "=r"(b[11]), "=r"(b[12]), "=r"(b[13]), "=r"(b[14]), "=r"(b[15])
+                        : "=r"(a[d][0]), "=r"(a[d][1]), "=r"(a[d][2]), "=r"(a[d][3]), "=r"(a[d][4]), "=r"(a[d][5]), "=r"(a[d][6]), "=r"(a[d][7]),
+                          "=r"(a[d][8]), "=r"(a[d][9]), "=r"(a[d][10]), "=r"(a[d][11]), "=r"(a[d][12]), "=r"(a[d][13]), "=r"(a[d][14]), "=r"(a[d][15])
                         : "r"(taddr));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                }
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                long long t[16];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) a[d][i] += b[i];   // the four k4 chains of this digit plane
+                for (int i = 0; i < 16; ++i) t[i] = digits_sum((int)a[2][i], (int)a[1][i], (int)a[0][i]);
+                if (whole) {
+                    finish(t);
+                } else {   // (all 16 rows of the place: the ones beyond M are never read into a result)
+                    long long* mine = sk.ws + ((size_t)blockIdx.x * 2 + (tile == tile0 ? 0 : 1)) * kPlace + (size_t)m0 * kGemmBN + col;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) __stcg(mine + (size_t)i * kGemmBN, t[i]);
                 }
             }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int m = m0 + i;
-                const long long t = ((long long)(int)a[2][i] << 16) + ((long long)(int)a[1][i] << 8) + (long long)(int)a[0][i];
-                if (m < g.M && n_ok) {
-                    if (S == 1) finish(m, t);
-                    else atomicAdd(sk.ws + (size_t)m * sk.n_pad + n, (unsigned long long)t);
-                }
-            }
-        }
-        if (S > 1) {
-            __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            if (whole) continue;
+            bar_sync(1, 32 * kSmallEpiWarps);
             if (threadIdx.x == 0) {
-                const unsigned int prev = atomicAdd(sk.cnt + nb, 1u);
-                *flag = prev == (unsigned int)(S - 1) ? 1 : 0;
-                if (*flag) sk.cnt[nb] = 0u;
+                fence_acq_rel_gpu();   // (the other warps' partial sums are ordered before this by the barrier)
+                const unsigned int prev = atomicAdd(sk.cnt + tile, 1u);
+                *flag = prev == (unsigned int)(c1 - c0) ? 1 : 0;
+                if (*flag) sk.cnt[tile] = 0u;
+                fence_acq_rel_gpu();
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (*flag) {   // every split of this tile has added its partial sums
-                __threadfence();
-                for (int m0 = 0; m0 < g.M; m0 += 16) {   // 16 loads in flight, then their 16 rows
-                    unsigned long long v[16];
+            bar_sync(1, 32 * kSmallEpiWarps);
+            if (*flag && ok && active) {
+                long long t[16];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = (m0 + i < g.M && n_ok) ? __ldcg(sk.ws + (size_t)(m0 + i) * sk.n_pad + n) : 0ull;
+                for (int i = 0; i < 16; ++i) t[i] = 0;
+                for (int c = c0; c <= c1; ++c) {
+                    const long long* p = sk.ws + ((size_t)c * 2 + (small_unit(units, c, ctas) / KB == tile ? 0 : 1)) * kPlace + (size_t)m0 * kGemmBN + col;
+                    long long v[16];   // (all requested before the first is added)
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (m0 + i < g.M && n_ok) {
-                            finish(m0 + i, (long long)v[i]);
-                            sk.ws[(size_t)(m0 + i) * sk.n_pad + n] = 0ull;
-                        }
+                    for (int i = 0; i < 16; ++i) v[i] = __ldcg(p + (size_t)i * kGemmBN);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) t[i] += v[i];
                 }
+                finish(t);
             }
         }
-        if (sk.dbg && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) sk.dbg[2] = clock64();
         tc_fence_before();
     }
     __syncthreads();
-    if (warp == 4) {
+    if (warp == 8) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kSmallTmemCols) : "memory");
     }

@@ -71,11 +71,13 @@ __global__ void rmsnorm_digits_kernel(const float* x, const float* w, float eps,
     }
 }
 
-// qkv[M][3H] (q | k | v) -> RoPE on q (in place) and k, k / v rows appended to the paged cache at positions pos0 + m
-__global__ void rope_kv_kernel(float* qkv, int M, int H, int rope_dim, const float* inv_freq, int pos0, float* k_pool, float* v_pool,
-                               const int* page_table, int page_tokens) {
+// qkv[M][3H] (q | k | v) -> RoPE on q (in place) and k, k / v rows appended to the paged cache.  The M rows are the first P positions of
+// M / P sequences, one after another, sequence i's page table at page_table + i * pages_per_seq
+__global__ void rope_kv_kernel(float* qkv, int P, int H, int rope_dim, const float* inv_freq, float* k_pool, float* v_pool, const int* page_table, int pages_per_seq,
+                               int page_tokens) {
     const int m = blockIdx.x;
-    const int pos = pos0 + m;
+    const int pos = m % P;
+    page_table += (size_t)(m / P) * pages_per_seq;
     float* row = qkv + (size_t)m * 3 * H;
     const int page = page_table[pos / page_tokens];
     const size_t kvoff = ((size_t)page * page_tokens + (pos % page_tokens)) * H;
@@ -427,28 +429,33 @@ __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t saddr) 
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr));
 }
 // ---- the default attention of the prefill, head dimensions 64 and 128: attn_tc.cuh over the paged cache (which already holds the rows' own K / V)
-struct PrefillKeys {   // kv_images_kernel: key t of the prompt
+struct PrefillKeys {   // kv_images_kernel: key t of a prompt; the prompts (P tokens each) one after another, kt tiles a prompt
     const float *k_pool, *v_pool;
     const int* page_table;
-    int page_tokens, H, d, dv, n, g0;
-    struct Tile { int t0; };
-    __device__ bool tile(int x, Tile& t) const { t.t0 = x * kAtKT; return true; }
+    int pages_per_seq, page_tokens, H, d, dv, P, kt, g0;
+    struct Tile { const int* table; int t0; };
+    __device__ bool tile(int x, Tile& t) const {
+        t.table = page_table + (size_t)(x / kt) * pages_per_seq;
+        t.t0 = x % kt * kAtKT;
+        return true;
+    }
     __device__ const float* row(const Tile& tile, int r, int g, bool is_v) const {
         const int t = tile.t0 + r;
-        if (t >= n) return nullptr;
-        return (is_v ? v_pool : k_pool) + ((size_t)page_table[t / page_tokens] * page_tokens + t % page_tokens) * H + (size_t)g * d;
+        if (t >= P) return nullptr;
+        return (is_v ? v_pool : k_pool) + ((size_t)tile.table[t / page_tokens] * page_tokens + t % page_tokens) * H + (size_t)g * d;
     }
 };
 struct PrefillAttn {
     const float* qkv;
     float* out;
-    int M, H, d, dv, group, h0, pos0;
+    int n_seq, P, kt, H, d, dv, group, h0;
     float scale;
     __device__ void tile(int y, int& row0, int& count, int& p0, int& image0) const {
-        row0 = (int)(gridDim.y - 1 - y) * kAtQ;   // latest queries (most key tiles) first: no long tail
-        count = min(kAtQ, M - row0);
-        p0 = pos0 + row0;
-        image0 = 0;
+        const int z = (int)(gridDim.y - 1 - y), seq = z % n_seq;
+        p0 = z / n_seq * kAtQ;   // latest queries (most key tiles) first: no long tail
+        row0 = seq * P + p0;
+        count = min(kAtQ, P - p0);
+        image0 = seq * kt;
     }
     __device__ const float* q(int row, int h) const { return qkv + (size_t)row * 3 * H + (size_t)h * d; }
     __device__ int first_key(int) const { return 0; }
