@@ -1096,7 +1096,7 @@ int ensure_kmajor(QWeight& w) {
     w.n_pad = (4 * w.L.U + kGemmBN - 1) / kGemmBN * kGemmBN;
     TRY(w.kmajor.alloc((size_t)w.n_pad * w.k_pad));
     CK(cudaMemsetAsync(w.kmajor.p, 0, (size_t)w.n_pad * w.k_pad, g_stream));
-    unpack_kmajor_kernel<<<w.L.P, kConsumerThreads, 0, g_stream>>>(w.packed.p, w.L, w.k_pad, w.kmajor.p);
+    unpack_kmajor_kernel<<<dim3(w.L.P, 4), kConsumerThreads, 0, g_stream>>>(w.packed.p, w.L, w.k_pad, w.kmajor.p);
     ++g_launches;
     CK(cudaGetLastError());
     return 0;

@@ -101,22 +101,25 @@ TIB_HD size_t sw128_offset(int row, int byte) {   // inside a tile whose rows ar
 TIB_HD size_t wtile_offset(int n, int k, int k_pad) {
     return ((size_t)(n / kGemmBN) * (k_pad / kGemmBK) + k / kGemmBK) * kGemmTileBytes + sw128_offset(n % kGemmBN, k % kGemmBK);
 }
-// packed streaming layout -> tile-major bytes, same thread mapping as unpack_kernel
+// packed streaming layout -> tile-major bytes, grid (slabs, parts), thread mapping of unpack_kernel.  A word of the packed layout is four
+// consecutive k of one column (INT8), or two such fours 32 k apart (INT4, low and high nibbles): whole words are stored (byte stores took four times as
+// long: 16 ms instead of 3 for 0.8 GB of INT8 weights, the first prompt of a model)
 __global__ void unpack_kmajor_kernel(const uint8_t* packed, QLayout L, int k_pad, uint8_t* wk) {
     const Slab slab = make_slab(L, blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kik = kitem_k(L.bits), nel = L.bits == 4 ? 8 : 4;
+    const int kik = kitem_k(L.bits);
     for_each_quad_word(L, slab, warp, lane, [&](size_t off, int nl, int grp, int chunk, int ki, int widx) {
         const uint32_t word = *reinterpret_cast<const uint32_t*>(packed + off);
-        for (int i = 0; i < nel; ++i) {
-            int row, kk;
-            kitem_word_elem(L.bits, nl, widx, i, row, kk);
-            const int n = slab.col0 + 16 * grp + row, k = chunk * L.kc + ki * kik + kk;
-            if (k >= k_pad) continue;
-            // INT4: u = q + woff (0..15); INT8: two's complement q
-            wk[wtile_offset(n, k, k_pad)] = (uint8_t)(L.bits == 4 ? (word >> (4 * i)) & 0xFu : (word >> (8 * i)) & 0xFFu);
+        int row, kk;
+        kitem_word_elem(L.bits, nl, widx, 0, row, kk);
+        const int n = slab.col0 + 16 * grp + row, k = chunk * L.kc + ki * kik + kk;   // (k and k_pad are multiples of four)
+        if (L.bits == 8) {   // two's complement q
+            if (k < k_pad) *reinterpret_cast<uint32_t*>(wk + wtile_offset(n, k, k_pad)) = word;
+        } else {             // u = q + woff (0..15)
+            if (k < k_pad) *reinterpret_cast<uint32_t*>(wk + wtile_offset(n, k, k_pad)) = word & 0x0F0F0F0Fu;
+            if (k + 32 < k_pad) *reinterpret_cast<uint32_t*>(wk + wtile_offset(n, k + 32, k_pad)) = (word >> 4) & 0x0F0F0F0Fu;
         }
-    });
+    }, blockIdx.y, gridDim.y);
 }
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------------

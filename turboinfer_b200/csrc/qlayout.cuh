@@ -140,16 +140,19 @@ TIB_HD void kitem_word_elem(int bits, int nl, int widx, int i, int& row, int& kk
 #ifdef __CUDACC__
 // Walks the 32-bit words of the quads that consumer warp `warp` of slab `slab` owns (the pack / unpack kernels mirror
 // the GEMV's 16 consumer warps): f(byte offset of the word in the packed buffer, nl, group, chunk, k-item, word in k-item)
+// (parts > 1: the rounds are dealt to that many callers, this one is number `part`)
 template <typename F>
-__device__ __forceinline__ void for_each_quad_word(const QLayout& L, const Slab& slab, int warp, int lane, F&& f) {
+__device__ __forceinline__ void for_each_quad_word(const QLayout& L, const Slab& slab, int warp, int lane, F&& f, int part = 0, int parts = 1) {
     const int nq = warp_quads(slab, warp), fq = warp_first_quad(slab, warp);
     size_t stage_base = 0;    // byte offset of round r inside the slab
     for (int r = 0; r < nq; ++r) {
+        const size_t round0 = slab.byte0 + stage_base;
+        stage_base += (size_t)round_total(slab, r) * kItemBytes;
+        if (parts > 1 && r % parts != part) continue;
         const int q = fq + r;
         const int grp = q / L.nchunks, chunk = q - grp * L.nchunks;
         const int nl = q >= slab.qfull ? slab.nlast : 4;
-        const size_t qoff = slab.byte0 + stage_base + (size_t)round_warp_offset(slab, r, warp) * kItemBytes;
-        stage_base += (size_t)round_total(slab, r) * kItemBytes;
+        const size_t qoff = round0 + (size_t)round_warp_offset(slab, r, warp) * kItemBytes;
         const int wpk = nl * 32;   // words per k-item
         for (int wq = lane; wq < 4 * wpk; wq += 32) f(qoff + (size_t)wq * 4, nl, grp, chunk, wq / wpk, wq % wpk);
     }
