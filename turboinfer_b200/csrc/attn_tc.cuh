@@ -14,9 +14,12 @@
 //   warp 0       producer: bulk copies of the key and value halves of a tile into two stages each
 //   warp 1       tcgen05.mma: S(i + 1) = Q K^T is issued before P(i) V, so that the scores of the next tile are made while the softmax of
 //                this one runs; S and the tile outputs P V have two TMEM buffers each (2 x 64 + 2 x DV columns)
-//   warps 2..5   softmax, one thread a row (no shuffles): scores from TMEM, masks, running maximum, expf, halves of P to shared memory
-//   warps 6..9   running output in registers, one thread a row: o = o * factor(i) + (P V)(i); then the finish (denominator, gates) and
-//                stores of whole 128-byte lines
+//   warps 4..11  softmax, two threads a row with 32 keys each (they exchange their maxima through shared memory): scores from TMEM, masks, running
+//                maximum, expf, halves of P to shared memory
+//   warps 12..15 running output in registers, one thread a row: o = o * factor(i) + (P V)(i); then the finish (denominator, gates) and
+//                stores of whole 128-byte lines; they take the registers that the others give back (80 + 112 + 112 + 208 = 4 x 128)
+// What bounds it: per tile of 64 keys 36 MMAs (1920 clocks: the scores' operand reads limit them) against the softmax's issue slots; with one
+// thread a row (four warps) the softmax took 4800 clocks a tile.
 // Waits are bounded; a wait that runs out sets *err and nothing is stored.
 #pragma once
 #include <cuda_fp16.h>
@@ -25,11 +28,11 @@
 
 namespace tib {
 
-constexpr int kAtQ = 128, kAtKT = 64, kAtThreads = 320;
+constexpr int kAtQ = 128, kAtKT = 64, kAtHalf = kAtKT / 2, kAtThreads = 512;
 __host__ __device__ constexpr int at_pad(int d) { return d <= 64 ? 64 : 128; }
 __host__ __device__ constexpr size_t at_record_bytes(int dk, int dv) { return (size_t)kAtKT * (dk + dv) * 4; }   // hi and lo of 64 rows
 template <int DK, int DV> constexpr size_t attn_tc_smem_bytes5() {
-    return (size_t)kAtQ * DK * 4 + 2 * at_record_bytes(DK, DV) + (size_t)kAtQ * kAtKT * 4 + 4 * kAtQ * sizeof(float) + 256;
+    return (size_t)kAtQ * DK * 4 + 2 * at_record_bytes(DK, DV) + (size_t)kAtQ * kAtKT * 4 + 5 * kAtQ * sizeof(float) + 256;
 }
 
 __device__ __forceinline__ void split_half(float x, float y, uint32_t& hi, uint32_t& lo) {   // two neighbours, packed
@@ -88,7 +91,7 @@ __device__ __forceinline__ void tc_mma_f16_if(uint32_t tmem_d, uint64_t adesc, u
 }
 // Shape: tile(y, row0, count, pos0, image0) -- the rows of the block, the position of the first, the record of the sequence's key tile 0;
 // d, dv (multiples of four), h0 (first query head of the launch), group (query heads a key/value head); q(row, h); first_key(pos), never
-// later for an earlier row; scores(): scales (and caps) raw products; sigmoid(): weights sigmoid_weight(score, pb(h)) instead of a softmax;
+// later for an earlier row; scores(): scales (and caps) 32 raw products; sigmoid(): weights sigmoid_weight(score, pb(h)) instead of a softmax;
 // finish(row, h, m, l): factor on the output; store4(row, h, c, v)
 template <int DK, int DV, typename Shape>
 __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, const uint8_t* images, int* err) {
@@ -99,13 +102,14 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
     uint8_t* Ks = Q + 2 * kQ;                                    // [2 stages][hi | lo]
     uint8_t* Vs = Ks + 4 * kK;
     uint8_t* P = Vs + 4 * kV;                                    // [hi | lo], 128 rows of 64 keys
-    float* factor = reinterpret_cast<float*>(P + kAtQ * kAtKT * 4);   // [4][128]: what the running output is multiplied by in front of tile i
-    uint64_t* bars = reinterpret_cast<uint64_t*>(factor + 4 * kAtQ);
+    float* factor = reinterpret_cast<float*>(P + kAtQ * kAtKT * 4);   // [3][128]: what the running output is multiplied by in front of tile i
+    float* pmax = factor + 3 * kAtQ;                             // [2][128]: the maxima of the two halves of a row's keys
+    uint64_t* bars = reinterpret_cast<uint64_t*>(pmax + 2 * kAtQ);
     uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 6, *s_full = bars + 8, *s_empty = bars + 10, *o_full = bars + 12,
              *o_empty = bars + 14, *p_full = bars + 16, *p_empty = bars + 17, *fin_full = bars + 18;
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 19);
     // behind the last tile the key stages hold what the rows end with, and the blocks of the store
-    float* fin = reinterpret_cast<float*>(Ks);                   // [m: 128][l: 128]
+    float* fin = reinterpret_cast<float*>(Ks);                   // [m: 128][l of either half: 2 x 128]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = s.h0 + blockIdx.x, groups = gridDim.x / s.group;   // (the launch covers whole key/value heads from h0 on)
     int row0, M, pos0, image0;
@@ -115,9 +119,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-            mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); mbar_init(&o_full[i], 1); mbar_init(&o_empty[i], 4);
+            mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 8); mbar_init(&o_full[i], 1); mbar_init(&o_empty[i], 4);
         }
-        mbar_init(p_full, 4); mbar_init(p_empty, 1); mbar_init(fin_full, 4);
+        mbar_init(p_full, 8); mbar_init(p_empty, 1); mbar_init(fin_full, 8);
         fence_mbar_init();
         if (smem_u32(at_smem) & 1023u) *reinterpret_cast<volatile int*>(err) = 1;   // (the swizzle needs 1024-byte blocks)
     }
@@ -151,7 +155,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
     const uint32_t tmem = *tmem_ptr;
     constexpr uint32_t kSCol = 0, kOCol = 2 * kAtKT;             // TMEM columns: two score buffers, two output buffers
 
+    // (the registers move inside the roles' own branches: the compiler allots each branch by it)
     if (warp == 0) {
+        reg_dealloc<80>();
         const uint32_t lead = elect_one();
         const uint8_t* rec = images + ((size_t)(image0 + first) * groups + blockIdx.x / s.group) * at_record_bytes(DK, DV);
         const size_t step = (size_t)groups * at_record_bytes(DK, DV);
@@ -169,6 +175,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
         if (!ok)
             for (int st = 0; st < 2; ++st) { mbar_wait_bounded(&k_full[st], 0, err); mbar_wait_bounded(&v_full[st], 0, err); }
     } else if (warp == 1) {
+        reg_dealloc<80>();
         const uint32_t lead = elect_one();
         constexpr uint32_t id_s = umma_idesc_f16(kAtQ, kAtKT, 0), id_o = umma_idesc_f16(kAtQ, DV, 1);
         const uint64_t qd = umma_desc_sw128(smem_u32(Q)), kd0 = umma_desc_sw128(smem_u32(Ks)), pd = umma_desc_sw128(smem_u32(P));
@@ -214,47 +221,53 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
             tc_commit_if(smem_u32(&v_empty[b]), lead);
             tc_commit_if(smem_u32(&o_full[b]), lead);
         }
-    } else if (warp < 6) {
-        const int q = warp & 3, r = q * 32 + lane;   // TMEM lane = row of the tile
+    } else if (warp < 4) {
+        reg_dealloc<80>();
+    } else if (warp < 12) {
+        reg_dealloc<112>();
+        const int q = warp & 3, r = q * 32 + lane, half = (warp - 4) >> 2, k0 = half * kAtHalf;   // TMEM lane = row of the tile
         const int qp = r < M ? pos0 + r : -1, lo = r < M ? s.first_key(pos0 + r) : 0;
         const int all_hi = M == kAtQ ? pos0 : -1, all_lo = s.first_key(last_pos);   // keys in [all_lo, all_hi] are visible to every row of the tile
         const float pb = s.sigmoid() ? s.pb(h) : 0.f;
         float m = -INFINITY, l = 0.f;
         bool ok = true;
-        for (int i = 0; i < n_tiles; ++i) {
+        // (after a failed wait the loop goes on without waiting: the two warps of a row meet at the same barriers to the end)
+        for (int i = 0, slot = 0; i < n_tiles; ++i, slot = slot == 2 ? 0 : slot + 1) {
             const int b = i & 1, use = i >> 1;
-            ok = mbar_wait_bounded(&s_full[b], use & 1, err);
+            if (ok) ok = mbar_wait_bounded(&s_full[b], use & 1, err);
             ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
             tc_fence_after();
-            uint32_t raw[2][32];
-            tmem_ld32(raw[0], tmem + ((uint32_t)(q * 32) << 16) + kSCol + b * kAtKT);
-            tmem_ld32(raw[1], tmem + ((uint32_t)(q * 32) << 16) + kSCol + b * kAtKT + 32);
+            uint32_t raw[kAtHalf];
+            tmem_ld32(raw, tmem + ((uint32_t)(q * 32) << 16) + kSCol + b * kAtKT + k0);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_empty[b]);
-            float sc[kAtKT];
+            float sc[kAtHalf];
 #pragma unroll
-            for (int j = 0; j < kAtKT; ++j) sc[j] = __uint_as_float(raw[j >> 5][j & 31]);
+            for (int j = 0; j < kAtHalf; ++j) sc[j] = __uint_as_float(raw[j]);
             s.scores(sc);
             const int t0 = (first + i) * kAtKT;
             if (!(t0 >= all_lo && t0 + kAtKT - 1 <= all_hi)) {
 #pragma unroll
-                for (int j = 0; j < kAtKT; ++j) sc[j] = (t0 + j <= qp && t0 + j >= lo) ? sc[j] : -INFINITY;
+                for (int j = 0; j < kAtHalf; ++j) sc[j] = (t0 + k0 + j <= qp && t0 + k0 + j >= lo) ? sc[j] : -INFINITY;
             }
             float f = 1.f;
             if (s.sigmoid()) {   // no softmax: a visible key's weight is sigmoid(score + pb)
 #pragma unroll
-                for (int j = 0; j < kAtKT; ++j) sc[j] = sc[j] == -INFINITY ? 0.f : s.sigmoid_weight(sc[j], pb);
+                for (int j = 0; j < kAtHalf; ++j) sc[j] = sc[j] == -INFINITY ? 0.f : s.sigmoid_weight(sc[j], pb);
             } else {
                 float mx[4] = {sc[0], sc[1], sc[2], sc[3]};
 #pragma unroll
-                for (int j = 4; j < kAtKT; ++j) mx[j & 3] = fmaxf(mx[j & 3], sc[j]);
-                const float mn = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
+                for (int j = 4; j < kAtHalf; ++j) mx[j & 3] = fmaxf(mx[j & 3], sc[j]);
+                const float mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                pmax[half * kAtQ + r] = mine;
+                bar_sync(2 + q, 64);
+                const float mn = fmaxf(m, fmaxf(mine, pmax[(half ^ 1) * kAtQ + r]));
+                bar_sync(2 + q, 64);   // (both have read: the place is free for the next tile)
                 const float base = mn == -INFINITY ? 0.f : mn;   // (nothing visible so far: exp(-inf) = 0 everywhere)
                 float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int j = 0; j < kAtKT; ++j) {
+                for (int j = 0; j < kAtHalf; ++j) {
                     sc[j] = expf(sc[j] - base);
                     sum[j & 3] += sc[j];
                 }
@@ -262,44 +275,44 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
                 l = l * f + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
                 m = mn;
             }
-            if (i > 0) ok = mbar_wait_bounded(p_empty, (i - 1) & 1, err);   // the previous tile's P V has read the halves
+            if (ok && i > 0) ok = mbar_wait_bounded(p_empty, (i - 1) & 1, err);   // the previous tile's P V has read the halves
             ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
 #pragma unroll
-            for (int c = 0; c < kAtKT / 8; ++c) {
+            for (int c = 0; c < kAtHalf / 8; ++c) {
                 uint4 hi, lo4;
                 split_half(sc[8 * c], sc[8 * c + 1], hi.x, lo4.x);
                 split_half(sc[8 * c + 2], sc[8 * c + 3], hi.y, lo4.y);
                 split_half(sc[8 * c + 4], sc[8 * c + 5], hi.z, lo4.z);
                 split_half(sc[8 * c + 6], sc[8 * c + 7], hi.w, lo4.w);
-                const uint32_t at = at_offset(kAtQ, r, 8 * c);
+                const uint32_t at = at_offset(kAtQ, r, k0 + 8 * c);
                 *reinterpret_cast<uint4*>(P + at) = hi;
                 *reinterpret_cast<uint4*>(P + kAtQ * kAtKT * 2 + at) = lo4;
             }
-            factor[(i & 3) * kAtQ + r] = f;   // (four slots: the output warps are at most two tiles behind)
+            if (half == 0) factor[slot * kAtQ + r] = f;   // (three slots: the output warps are at most two tiles behind)
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full);
         }
         if (ok) {   // (every S has been made: the key stages are free)
-            fin[r] = m;
-            fin[kAtQ + r] = l;
+            if (half == 0) fin[r] = m;
+            fin[(1 + half) * kAtQ + r] = l;
             __syncwarp();
             if (lane == 0) mbar_arrive(fin_full);
         }
     } else {
+        reg_alloc<208>();
         const int q = warp & 3, r = q * 32 + lane;
         float o[DV];
 #pragma unroll
         for (int c = 0; c < DV; ++c) o[c] = 0.f;
         bool ok = true;
-        for (int i = 0; i < n_tiles; ++i) {
+        for (int i = 0, slot = 0; i < n_tiles; ++i, slot = slot == 2 ? 0 : slot + 1) {
             const int b = i & 1, use = i >> 1;
             ok = mbar_wait_bounded(&o_full[b], use & 1, err);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const float f = factor[(i & 3) * kAtQ + r];
+            const float f = factor[slot * kAtQ + r];
 #pragma unroll
             for (int c = 0; c < DV; c += 32) {
                 uint32_t v[32];
@@ -314,8 +327,8 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
         if (ok) ok = mbar_wait_bounded(fin_full, 0, err);
         ok = __all_sync(0xffffffffu, ok);
         if (ok) {
-            const float fac = r < M ? s.finish(row0 + r, h, fin[r], fin[kAtQ + r]) : 0.f;
-            float* blk = reinterpret_cast<float*>(Ks + 1024) + (warp - 6) * (32 * 36);
+            const float fac = r < M ? s.finish(row0 + r, h, fin[r], fin[kAtQ + r] + fin[2 * kAtQ + r]) : 0.f;
+            float* blk = reinterpret_cast<float*>(Ks + 2048) + (warp - 12) * (32 * 36);
             const int rr = lane >> 3, cc = 4 * (lane & 7);
 #pragma unroll
             for (int c = 0; c < DV; c += 32) {

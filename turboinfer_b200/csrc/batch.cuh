@@ -38,25 +38,37 @@ __global__ void rope_kv_batch_kernel(float* qkv, int H, int rope_dim, const floa
     }
 }
 
-// rmsnorm_digits_kernel for the batched decode: one block of 1024 threads per row, the row stays in registers between the
-// passes (K <= 16384), the digit planes are written four bytes at a time.  gu != nullptr: the row is not read from x but
-// computed on the fly as up * silu(gate) from the interleaved (gate_i, up_i) columns of gu[M][2K] (SwiGLU fused in front
-// of the down projection, :918, :1729).  Same expressions as rmsnorm_digits_kernel (prefill.cuh).
-constexpr int kDigitsThreads = 1024, kDigitsVecs = 4;   // 4 float4 per thread
-// tile_layout = 16 or 32: planes in the few-row GEMM's tile images of so many rows (xtile_offset); 0: [3][m_pad][k_pad] row-major for the 128-row GEMM
+// rmsnorm_digits_kernel with the row in registers between the passes (K <= 16384): one block per row, sixteen values a thread at most, the
+// digit planes written four bytes at a time.  gu != nullptr: the row is not read from x but computed on the fly as up * silu(gate) from the
+// interleaved (gate_i, up_i) columns of gu[M][2K] (SwiGLU fused in front of the down projection, :918, :1729).  Same expressions as
+// rmsnorm_digits_kernel (prefill.cuh).
+// Threads (digits_threads): few rows are a matter of latency, 1024 threads a row; from a row per SM on the rows are a matter of bandwidth, and a thread
+// takes its full sixteen values so that several rows share an SM (2047 rows of 4096 behind a norm, us: 52 with 1024 threads a row, 20 with 256; 332 rows of
+// 2048: 12 and 7).
+constexpr int kDigitsThreads = 1024, kDigitsVecs = 4;   // most threads a row; 4 float4 per thread
+inline int digits_threads(int rows, int k_pad, int sms) {
+    return rows <= sms ? kDigitsThreads : std::min(kDigitsThreads, std::max(128, ((k_pad + 4 * kDigitsVecs - 1) / (4 * kDigitsVecs) + 31) / 32 * 32));
+}
+// tile_layout = 16 or 32: planes in the few-row GEMM's tile images of so many rows (xtile_offset); 0: [3][m_pad][k_pad] row-major for the pair GEMM
 __global__ void __launch_bounds__(kDigitsThreads) rmsnorm_digits_small_kernel(const float* x, const float* gu, const float* w, float eps, int K,
                                                                                int m_pad, int k_pad, int8_t* planes, float* sx_out, long long* sxf_out,
                                                                                int tile_layout) {
+    __shared__ float red[2][32];
+    __shared__ long long redl[32];
+    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+    float4 v[kDigitsVecs], ww[kDigitsVecs];
+#pragma unroll
+    for (int i = 0; i < kDigitsVecs; ++i) {   // (the gains do not depend on the kernel before: they are on their way while it ends)
+        const int k = 4 * (tid + i * nt);
+        ww[i] = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (w && k < K) ww[i] = *reinterpret_cast<const float4*>(w + k);
+    }
     pdl_wait_prior_grid();       // (no-op unless launched with programmatic stream serialization: the lockstep step's graph)
     pdl_launch_dependents();
-    __shared__ float red[32];
-    __shared__ long long redl[32];
-    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    float4 v[kDigitsVecs];
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < kDigitsVecs; ++i) {
-        const int k = 4 * (tid + i * kDigitsThreads);
+        const int k = 4 * (tid + i * nt);
         v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (k < K) {
             if (gu) {
@@ -68,40 +80,33 @@ __global__ void __launch_bounds__(kDigitsThreads) rmsnorm_digits_small_kernel(co
                 v[i] = *reinterpret_cast<const float4*>(x + (size_t)row * K + k);
             }
         }
-        ss = fmaf(v[i].x, v[i].x, ss); ss = fmaf(v[i].y, v[i].y, ss); ss = fmaf(v[i].z, v[i].z, ss); ss = fmaf(v[i].w, v[i].w, ss);
     }
+#pragma unroll
+    for (int i = 0; i < kDigitsVecs; ++i) { ss = fmaf(v[i].x, v[i].x, ss); ss = fmaf(v[i].y, v[i].y, ss); ss = fmaf(v[i].z, v[i].z, ss); ss = fmaf(v[i].w, v[i].w, ss); }
     float amax = 0.f;
     if (w) {
         ss = warp_sum(ss);
-        if (lane == 0) red[wid] = ss;
+        if (lane == 0) red[0][wid] = ss;
         __syncthreads();
-        float tot = 0.f;
-        for (int i = 0; i < kDigitsThreads / 32; ++i) tot += red[i];
-        __syncthreads();
+        const float tot = warp_sum(lane < nw ? red[0][lane] : 0.f);
         const float rms = sqrtf(tot / (float)K + eps);   // :1501
 #pragma unroll
-        for (int i = 0; i < kDigitsVecs; ++i) {
-            const int k = 4 * (tid + i * kDigitsThreads);
-            if (k < K) {
-                const float4 ww = *reinterpret_cast<const float4*>(w + k);
-                v[i] = make_float4((v[i].x / rms) * ww.x, (v[i].y / rms) * ww.y, (v[i].z / rms) * ww.z, (v[i].w / rms) * ww.w);   // :1504-1506
-            }
-        }
+        for (int i = 0; i < kDigitsVecs; ++i)
+            if (4 * (tid + i * nt) < K) v[i] = make_float4((v[i].x / rms) * ww[i].x, (v[i].y / rms) * ww[i].y, (v[i].z / rms) * ww[i].z, (v[i].w / rms) * ww[i].w);   // :1504-1506
     }
 #pragma unroll
     for (int i = 0; i < kDigitsVecs; ++i) amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
     amax = warp_max(amax);
-    if (lane == 0) red[wid] = amax;
+    if (lane == 0) red[1][wid] = amax;
     __syncthreads();
-    amax = 0.f;
-    for (int i = 0; i < kDigitsThreads / 32; ++i) amax = fmaxf(amax, red[i]);
+    amax = warp_max(lane < nw ? red[1][lane] : 0.f);
     const bool finite = amax > 0.f && amax < INFINITY;
     const float inv_s = finite ? kXQMax / amax : 0.f;
     const float s_x = finite ? amax / kXQMax : 0.f;
     long long sxf = 0;
 #pragma unroll
     for (int i = 0; i < kDigitsVecs; ++i) {
-        const int k = 4 * (tid + i * kDigitsThreads);
+        const int k = 4 * (tid + i * nt);
         if (k < k_pad) {   // columns K .. k_pad - 1 are zero
             const int f0 = __float2int_rn(v[i].x * inv_s), f1 = __float2int_rn(v[i].y * inv_s), f2 = __float2int_rn(v[i].z * inv_s),
                       f3 = __float2int_rn(v[i].w * inv_s);
@@ -112,7 +117,7 @@ __global__ void __launch_bounds__(kDigitsThreads) rmsnorm_digits_small_kernel(co
             const uint32_t hi01 = __byte_perm(u0, u1, 0x0062), hi23 = __byte_perm(u2, u3, 0x0062);
             const uint32_t d0 = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u, d1 = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u,
                            d2 = __byte_perm(hi01, hi23, 0x5410) ^ 0x80808080u;
-            if (tile_layout) {   // the swizzled tile images the 32-row GEMM copies in bulk (gemm_tc.cuh xtile_offset)
+            if (tile_layout) {   // the swizzled tile images the few-row GEMM copies in bulk (gemm_tc.cuh xtile_offset)
                 *reinterpret_cast<uint32_t*>(planes + xtile_offset(0, row, k, tile_layout)) = d0;
                 *reinterpret_cast<uint32_t*>(planes + xtile_offset(1, row, k, tile_layout)) = d1;
                 *reinterpret_cast<uint32_t*>(planes + xtile_offset(2, row, k, tile_layout)) = d2;
@@ -127,11 +132,14 @@ __global__ void __launch_bounds__(kDigitsThreads) rmsnorm_digits_small_kernel(co
     for (int o = 16; o > 0; o >>= 1) sxf += __shfl_xor_sync(0xffffffffu, sxf, o);
     if (lane == 0) redl[wid] = sxf;
     __syncthreads();
-    if (tid == 0) {
-        long long t = 0;
-        for (int i = 0; i < kDigitsThreads / 32; ++i) t += redl[i];
-        sx_out[row] = s_x;
-        sxf_out[row] = t;
+    if (wid == 0) {
+        long long t = lane < nw ? redl[lane] : 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) {
+            sx_out[row] = s_x;
+            sxf_out[row] = t;
+        }
     }
 }
 
@@ -148,12 +156,19 @@ __global__ void argmax_rows_kernel(const float* logits, int V, int* tokens, int*
     const int b = blockIdx.x;
     const float* row = logits + (size_t)b * V;
     unsigned long long key = 0ull;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        // NaN never wins and -inf never beats "nothing yet" (key 0 -> token 0): the policy of the GEMV epilogue (`y > best`)
-        const float v = row[i];
+    // NaN never wins and -inf never beats "nothing yet" (key 0 -> token 0): the policy of the GEMV epilogue (`y > best`)
+    auto take = [&](float v, int i) {
         const unsigned long long k = v > -INFINITY ? argmax_pack(v, i) : 0ull;
         key = k > key ? k : key;
+    };
+    // 16-byte loads, four in flight a thread (a row of 32000: 18.7 us with one 4-byte load in flight)
+    const int v4 = (V & 3) == 0 ? V / 4 : 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < v4; i += blockDim.x) {
+        const float4 v = *reinterpret_cast<const float4*>(row + 4 * i);
+        take(v.x, 4 * i); take(v.y, 4 * i + 1); take(v.z, 4 * i + 2); take(v.w, 4 * i + 3);
     }
+    for (int i = 4 * v4 + threadIdx.x; i < V; i += blockDim.x) take(row[i], i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);

@@ -1220,7 +1220,7 @@ int pf_digits(Model& m, const float* x, const float* norm_w, int M, int K, int m
     if (pf_digits_fast(K, k_pad)) {
         // register-resident conversion, 4-byte stores; it writes every column < k_pad of the rows < M, and rows >= M only
         // produce output rows nobody stores: nothing to clear
-        rmsnorm_digits_small_kernel<<<M, kDigitsThreads, 0, g_stream>>>(x, gu, norm_w, m.cfg.rms_eps, K, m_pad, k_pad, m.pf_planes.p, m.pf_sx.p, m.pf_sxf.p, 0);
+        rmsnorm_digits_small_kernel<<<M, digits_threads(M, k_pad, g_num_sms), 0, g_stream>>>(x, gu, norm_w, m.cfg.rms_eps, K, m_pad, k_pad, m.pf_planes.p, m.pf_sx.p, m.pf_sxf.p, 0);
         ++g_launches;
         CK(cudaGetLastError());
         return 0;

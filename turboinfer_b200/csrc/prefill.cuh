@@ -459,9 +459,9 @@ struct PrefillAttn {
     }
     __device__ const float* q(int row, int h) const { return qkv + (size_t)row * 3 * H + (size_t)h * d; }
     __device__ int first_key(int) const { return 0; }
-    __device__ void scores(float (&s)[kAtKT]) const {
+    __device__ void scores(float (&s)[kAtHalf]) const {
 #pragma unroll
-        for (int j = 0; j < kAtKT; ++j) s[j] *= scale;
+        for (int j = 0; j < kAtHalf; ++j) s[j] *= scale;
     }
     __device__ bool sigmoid() const { return false; }
     __device__ float pb(int) const { return 0.f; }
@@ -487,7 +487,12 @@ __global__ void embed_rows_kernel(const float* emb, const int* tokens, float* x,
     pdl_launch_dependents();
     const int m = blockIdx.x;
     const float* e = emb + (size_t)tokens[m] * H;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) x[(size_t)m * H + i] = e[i];
+    if ((H & 3) == 0) {
+#pragma unroll 4
+        for (int i = 4 * threadIdx.x; i < H; i += 4 * blockDim.x) *reinterpret_cast<float4*>(x + (size_t)m * H + i) = *reinterpret_cast<const float4*>(e + i);
+    } else {
+        for (int i = threadIdx.x; i < H; i += blockDim.x) x[(size_t)m * H + i] = e[i];
+    }
 }
 
 }  // namespace tib

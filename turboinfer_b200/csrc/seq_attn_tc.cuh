@@ -50,14 +50,14 @@ struct SeqAttn {
     }
     __device__ const float* q(int row, int h) const { return qkvg + (size_t)row * s.ld + (size_t)h * d; }
     __device__ int first_key(int pos) const { return attn_first_key(s, pos); }
-    __device__ void scores(float (&v)[kAtKT]) const {
+    __device__ void scores(float (&v)[kAtHalf]) const {
         if (s.softcap > 0.f) {
             const float pre = s.scale / s.softcap;
 #pragma unroll
-            for (int j = 0; j < kAtKT; ++j) v[j] = s.softcap * tanhf(v[j] * pre);
+            for (int j = 0; j < kAtHalf; ++j) v[j] = s.softcap * tanhf(v[j] * pre);
         } else {
 #pragma unroll
-            for (int j = 0; j < kAtKT; ++j) v[j] *= s.scale;
+            for (int j = 0; j < kAtHalf; ++j) v[j] *= s.scale;
         }
     }
     __device__ bool sigmoid() const { return s.pb != nullptr; }
