@@ -11,7 +11,7 @@
 // k index of P V is the key).
 //
 // attn_tc_kernel: a CTA owns up to 128 query rows of one sequence and one head.
-//   warp 0       producer: bulk copies of the key and value halves of a tile into two stages each
+//   warps 0, 2   producers: bulk copies of the key and the value halves of a tile into two stages each
 //   warp 1       tcgen05.mma: S(i + 1) = Q K^T is issued before P(i) V, so that the scores of the next tile are made while the softmax of
 //                this one runs; S and the tile outputs P V have two TMEM buffers each (2 x 64 + 2 x DV columns)
 //   warps 4..11  softmax, two threads a row with 32 keys each (they exchange their maxima through shared memory): scores from TMEM, masks, running
@@ -111,12 +111,18 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
     // behind the last tile the key stages hold what the rows end with, and the blocks of the store
     float* fin = reinterpret_cast<float*>(Ks);                   // [m: 128][l of either half: 2 x 128]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = s.h0 + blockIdx.x, groups = gridDim.x / s.group;   // (the launch covers whole key/value heads from h0 on)
+    const int h = s.h0 + blockIdx.x;
     int row0, M, pos0, image0;
     s.tile(blockIdx.y, row0, M, pos0, image0);
     const int last_pos = pos0 + M - 1, first = s.first_key(pos0) / kAtKT, n_tiles = last_pos / kAtKT - first + 1;
 
-    if (threadIdx.x == 0) {
+    const int groups = gridDim.x / s.group;   // (the launch covers whole key/value heads from h0 on)
+    const uint8_t* rec0 = images + ((size_t)(image0 + first) * groups + blockIdx.x / s.group) * at_record_bytes(DK, DV);
+    const size_t step = (size_t)groups * at_record_bytes(DK, DV);
+    const uint32_t lead = elect_one();
+
+    if (warp == 0) {
+        if (lead) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
             mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 8); mbar_init(&o_full[i], 1); mbar_init(&o_empty[i], 4);
@@ -124,26 +130,48 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
         mbar_init(p_full, 8); mbar_init(p_empty, 1); mbar_init(fin_full, 8);
         fence_mbar_init();
         if (smem_u32(at_smem) & 1023u) *reinterpret_cast<volatile int*>(err) = 1;   // (the swizzle needs 1024-byte blocks)
+        }
+        __syncwarp();
+        // the first two key and value tiles are on their way while the query tile is split
+        for (int i = 0; i < 2 && i < n_tiles; ++i) {
+            mbar_expect_tx_if(smem_u32(&k_full[i]), 2 * kK, lead);
+            bulk_g2s_if(smem_u32(Ks) + i * 2 * kK, rec0 + i * step, 2 * kK, smem_u32(&k_full[i]), lead);
+            mbar_expect_tx_if(smem_u32(&v_full[i]), 2 * kV, lead);
+            bulk_g2s_if(smem_u32(Vs) + i * 2 * kV, rec0 + i * step + 2 * kK, 2 * kV, smem_u32(&v_full[i]), lead);
+        }
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_ptr)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // the query tile's halves
-    for (int i = threadIdx.x; i < kAtQ * DK / 8; i += kAtThreads) {
-        const int r = i / (DK / 8), d = (i % (DK / 8)) * 8;
-        float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (r < M) {
-            const float* q = s.q(row0 + r, h);   // (the row pitch need not be a multiple of 4)
+    // the query tile's halves, a thread's loads all in flight together
+    constexpr int kQVecs = kAtQ * DK / 8 / kAtThreads;
+    float x[kQVecs][8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (d + e < s.d) x[e] = q[d + e];
+    for (int i = 0; i < kQVecs; ++i) {
+        const int c = threadIdx.x + i * kAtThreads, r = c / (DK / 8), d = (c % (DK / 8)) * 8;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[i][e] = 0.f;
+        if (r < M) {
+            const float* q = s.q(row0 + r, h) + d;   // (the row pitch need not be a multiple of 4)
+            if ((reinterpret_cast<uintptr_t>(q) & 15) == 0) {
+                if (d < s.d) *reinterpret_cast<float4*>(x[i]) = *reinterpret_cast<const float4*>(q);
+                if (d + 4 < s.d) *reinterpret_cast<float4*>(x[i] + 4) = *reinterpret_cast<const float4*>(q + 4);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (d + e < s.d) x[i][e] = q[e];
+            }
         }
+    }
+#pragma unroll
+    for (int i = 0; i < kQVecs; ++i) {
+        const int c = threadIdx.x + i * kAtThreads, r = c / (DK / 8), d = (c % (DK / 8)) * 8;
         uint4 hi, lo;
-        split_half(x[0], x[1], hi.x, lo.x);
-        split_half(x[2], x[3], hi.y, lo.y);
-        split_half(x[4], x[5], hi.z, lo.z);
-        split_half(x[6], x[7], hi.w, lo.w);
+        split_half(x[i][0], x[i][1], hi.x, lo.x);
+        split_half(x[i][2], x[i][3], hi.y, lo.y);
+        split_half(x[i][4], x[i][5], hi.z, lo.z);
+        split_half(x[i][6], x[i][7], hi.w, lo.w);
         const uint32_t at = at_offset(kAtQ, r, d);
         *reinterpret_cast<uint4*>(Q + at) = hi;
         *reinterpret_cast<uint4*>(Q + kQ + at) = lo;
@@ -156,27 +184,21 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
     constexpr uint32_t kSCol = 0, kOCol = 2 * kAtKT;             // TMEM columns: two score buffers, two output buffers
 
     // (the registers move inside the roles' own branches: the compiler allots each branch by it)
-    if (warp == 0) {
+    if (warp == 0 || warp == 2) {   // keys, values
         reg_dealloc<80>();
-        const uint32_t lead = elect_one();
-        const uint8_t* rec = images + ((size_t)(image0 + first) * groups + blockIdx.x / s.group) * at_record_bytes(DK, DV);
-        const size_t step = (size_t)groups * at_record_bytes(DK, DV);
+        const bool is_v = warp == 2;
+        const uint32_t bytes = 2 * (is_v ? kV : kK), full = smem_u32(is_v ? v_full : k_full), dst = smem_u32(is_v ? Vs : Ks);
+        uint64_t* empty = is_v ? v_empty : k_empty;
+        const uint8_t* src = rec0 + (is_v ? 2 * kK : 0) + 2 * step;
         bool ok = true;
-        for (int i = 0; i < n_tiles && ok; ++i, rec += step) {
-            const int st = i & 1, use = i >> 1;
-            if (use > 0) ok = mbar_wait_bounded(&k_empty[st], (use - 1) & 1, err);
-            mbar_expect_tx_if(smem_u32(&k_full[st]), 2 * kK, lead);
-            bulk_g2s_if(smem_u32(Ks) + st * 2 * kK, rec, 2 * kK, smem_u32(&k_full[st]), lead);
-            if (use > 0 && ok) ok = mbar_wait_bounded(&v_empty[st], (use - 1) & 1, err);
-            mbar_expect_tx_if(smem_u32(&v_full[st]), 2 * kV, lead);
-            bulk_g2s_if(smem_u32(Vs) + st * 2 * kV, rec + 2 * kK, 2 * kV, smem_u32(&v_full[st]), lead);
+        for (int i = 2; i < n_tiles && ok; ++i, src += step) {   // (the first two tiles were asked for in front of the query tile)
+            const int st = i & 1;
+            ok = mbar_wait_bounded(&empty[st], ((i >> 1) - 1) & 1, err);
+            mbar_expect_tx_if(full + 8 * st, bytes, lead);
+            bulk_g2s_if(dst + st * bytes, src, bytes, full + 8 * st, lead);
         }
-        // (after a failed wait the copies issued so far are drained before the block ends)
-        if (!ok)
-            for (int st = 0; st < 2; ++st) { mbar_wait_bounded(&k_full[st], 0, err); mbar_wait_bounded(&v_full[st], 0, err); }
     } else if (warp == 1) {
         reg_dealloc<80>();
-        const uint32_t lead = elect_one();
         constexpr uint32_t id_s = umma_idesc_f16(kAtQ, kAtKT, 0), id_o = umma_idesc_f16(kAtQ, DV, 1);
         const uint64_t qd = umma_desc_sw128(smem_u32(Q)), kd0 = umma_desc_sw128(smem_u32(Ks)), pd = umma_desc_sw128(smem_u32(P));
         // values, MN-major: 64 coordinates a block (leading offset: the next block), 8 keys apart 1024 bytes
@@ -221,7 +243,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
             tc_commit_if(smem_u32(&v_empty[b]), lead);
             tc_commit_if(smem_u32(&o_full[b]), lead);
         }
-    } else if (warp < 4) {
+    } else if (warp == 3) {
         reg_dealloc<80>();
     } else if (warp < 12) {
         reg_dealloc<112>();
@@ -264,14 +286,15 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
                 bar_sync(2 + q, 64);
                 const float mn = fmaxf(m, fmaxf(mine, pmax[(half ^ 1) * kAtQ + r]));
                 bar_sync(2 + q, 64);   // (both have read: the place is free for the next tile)
-                const float base = mn == -INFINITY ? 0.f : mn;   // (nothing visible so far: exp(-inf) = 0 everywhere)
+                constexpr float kLog2e = 1.4426950408889634f;
+                const float base = mn == -INFINITY ? 0.f : mn * kLog2e;   // (nothing visible so far: exp(-inf) = 0 everywhere)
                 float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int j = 0; j < kAtHalf; ++j) {
-                    sc[j] = expf(sc[j] - base);
+                    sc[j] = exp2f(fmaf(sc[j], kLog2e, -base));
                     sum[j & 3] += sc[j];
                 }
-                f = mn == -INFINITY ? 1.f : expf(m - mn);
+                f = mn == -INFINITY ? 1.f : exp2f((m - mn) * kLog2e);
                 l = l * f + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
                 m = mn;
             }
