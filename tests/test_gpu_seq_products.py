@@ -47,3 +47,25 @@ def test_activated_columns(rows, heads, ff):
     m.free()
     want, _ = nubipel_plain.run(cfg, W, toks)
     assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+
+
+@pytest.mark.parametrize("dim", [32, 64, 128])
+@pytest.mark.parametrize("first,rows", [(0, 64), (0, 79), (5, 65), (33, 96), (70, 200)])
+def test_recurrence_in_chunks_equals_tokens(dim, first, rows):
+    """Portions of 64 rows and more run the wkv recurrence in chunks of 16 tokens, shorter ones token by token: the same rows both ways, from a
+    fresh state and behind earlier tokens, with a second request of its own length in the step."""
+    cfg = binusun_cases.make_config([binusun_cases.wkv_layer(heads=2, dim=dim, rank=8), binusun_cases.wkv_layer(heads=2, dim=dim, rank=8, ff=64)], width=64)
+    W = binusun_cases.random_weights(cfg, seed=first + rows, decay_bias=-2.0)
+    rng = np.random.default_rng(rows)
+    toks, other = [[int(t) for t in rng.integers(0, cfg["vocab"], n)] for n in (first + rows, 17)]
+    m = binusun_cases.build_engine(cfg, W, "float32")
+    s, o = m.open(), m.open()
+    got = []
+    if first:
+        got.append(m.step([(s, toks[:first])], [range(first)]))
+    both = m.step([(o, other), (s, toks[first:])], [range(17), range(rows)])
+    got.append(both[17:])
+    m.free()
+    # fp32 throughout; sums of up to 16 tokens and 128 channels in another order
+    for want, g in ((binusun_plain.forward(cfg, W, toks), np.concatenate(got)), (binusun_plain.forward(cfg, W, other), both[:17])):
+        assert np.abs(g - want).max() <= 2e-4 * np.abs(want).max()

@@ -9,7 +9,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libturboinfer_b200.so")
 SOURCES = ["capi.cu"]
-HEADERS = ["ptx.cuh", "qlayout.cuh", "gemv.cuh", "kernels.cuh", "mega.cuh", "gemm_tc.cuh", "attn_tc.cuh", "prefill.cuh", "batch.cuh", "sampling.cuh"]
+HEADERS = ["ptx.cuh", "qlayout.cuh", "gemv.cuh", "kernels.cuh", "mega.cuh", "gemm_tc.cuh", "attn_tc.cuh", "prefill.cuh", "batch.cuh", "sampling.cuh", "stage_out.cuh"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
          "-shared", "--expt-relaxed-constexpr", "-Xptxas", "-v"]
@@ -43,7 +43,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
 # quantized-decoder library to compile.
 SEQ_LIB = os.path.join(HERE, "libturboinfer_b200_seq.so")
 SEQ_SOURCES = ["seq_engine.cu"]
-SEQ_HEADERS = ["seq_kernels.cuh", "seq_headmix.cuh", "seq_hyper.cuh", "seq_ssm.cuh", "seq_delta.cuh", "seq_gemm_tc.cuh", "seq_attn_tc.cuh", "seq_recurrent.cuh", "seq_latent.cuh", "seq_experts.cuh", "prefill.cuh", "attn_tc.cuh", "gemm_tc.cuh", "sampling.cuh", "kernels.cuh", "gemv.cuh", "qlayout.cuh", "ptx.cuh"]
+SEQ_HEADERS = ["seq_kernels.cuh", "seq_wkv.cuh", "stage_out.cuh", "seq_headmix.cuh", "seq_hyper.cuh", "seq_ssm.cuh", "seq_delta.cuh", "seq_gemm_tc.cuh", "seq_attn_tc.cuh", "seq_recurrent.cuh", "seq_latent.cuh", "seq_experts.cuh", "prefill.cuh", "attn_tc.cuh", "gemm_tc.cuh", "sampling.cuh", "kernels.cuh", "gemv.cuh", "qlayout.cuh", "ptx.cuh"]
 
 
 def build_seq(force: bool = False) -> str:

@@ -21,6 +21,7 @@
 #include "gemm_tc.cuh"
 #include "prefill.cuh"
 #include "batch.cuh"
+#include "stage_out.cuh"
 #include "sampling.cuh"
 
 using namespace tib;
@@ -392,6 +393,7 @@ struct Model {
     int pf_cap = 0;
     float last_prefill_ms = 0.f;   // CUDA-event time of the prompt phase of the last generate call
     DevBuf<float> pf_x, pf_qkv, pf_attn, pf_gu, pf_act, pf_sx;
+    StageOut stage;              // logits on their way to the caller
     DevBuf<uint8_t> pf_images;   // split keys and values of the prefill attention
     DevBuf<int8_t> pf_planes;
     DevBuf<long long> pf_sxf;
@@ -2405,9 +2407,9 @@ int ti_b200_prefill(ti_model_t h, const int32_t* tokens, int32_t n, float* last_
             if (m.hist.n < V) TRY(m.hist.alloc(V));
             CK(cudaMemcpyAsync(m.hist.p, m.logits.p, V * 4, cudaMemcpyDeviceToDevice, g_stream));
             TRY(gather_sharded_logits(m, m.hist.p, V));
-            CK(cudaMemcpyAsync(last_logits_host, m.hist.p, V * 4, cudaMemcpyDeviceToHost, g_stream));
+            CK(m.stage.copy(last_logits_host, m.hist.p, V * 4, g_stream));
         } else {
-            CK(cudaMemcpyAsync(last_logits_host, m.logits.p, V * 4, cudaMemcpyDeviceToHost, g_stream));
+            CK(m.stage.copy(last_logits_host, m.logits.p, V * 4, g_stream));
         }
     }
     TRY(sync_stream());
@@ -2581,6 +2583,7 @@ int ti_b200_model_finalize(ti_model_t h) {
         TRY(capture_graph(m, true, &m.graph_decode));
         TRY(capture_graph(m, false, &m.graph_prefill));
     }
+    if (m.stage.open() != cudaSuccess) cudaGetLastError();   // (logits then take the driver's own way)
     m.finalized = true;
     m.host_pos = 0;
     return 0;
@@ -2674,9 +2677,9 @@ int ti_b200_decode_step(ti_model_t h, int32_t token, float* logits_host, int32_t
             if (m->hist.n < (size_t)m->cfg.vocab) TRY(m->hist.alloc((size_t)m->cfg.vocab));
             CK(cudaMemcpyAsync(m->hist.p, m->logits.p, (size_t)m->cfg.vocab * 4, cudaMemcpyDeviceToDevice, g_stream));
             TRY(gather_sharded_logits(*m, m->hist.p, (size_t)m->cfg.vocab));
-            CK(cudaMemcpyAsync(logits_host, m->hist.p, (size_t)m->cfg.vocab * 4, cudaMemcpyDeviceToHost, g_stream));
+            CK(m->stage.copy(logits_host, m->hist.p, (size_t)m->cfg.vocab * 4, g_stream));
         } else {
-            CK(cudaMemcpyAsync(logits_host, m->logits.p, (size_t)m->cfg.vocab * 4, cudaMemcpyDeviceToHost, g_stream));
+            CK(m->stage.copy(logits_host, m->logits.p, (size_t)m->cfg.vocab * 4, g_stream));
         }
     }
     int tok = 0;
@@ -2767,7 +2770,7 @@ int ti_b200_generate_greedy(ti_model_t h, const int32_t* prompt, int32_t n_promp
     if (have > 0) CK(cudaMemcpyAsync(toks.data(), m.out_tokens.p, have * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
     if (logits_host && have > 0) {
         TRY(gather_sharded_logits(m, m.hist.p, (size_t)have * V));
-        CK(cudaMemcpyAsync(logits_host, m.hist.p, (size_t)have * V * 4, cudaMemcpyDeviceToHost, g_stream));
+        CK(m.stage.copy(logits_host, m.hist.p, (size_t)have * V * 4, g_stream));
     }
     TRY(sync_stream());
     float ms = 0.f;
@@ -2916,7 +2919,7 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
     for (int i = 1; i < n_new; ++i) TRY(run(true));
     CK(cudaEventRecord(e1, g_stream));
     CK(cudaMemcpyAsync(out_tokens, bs.out.p, (size_t)B * n_new * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
-    if (logits_last) CK(cudaMemcpyAsync(logits_last, bs.logits.p, (size_t)B * V * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
+    if (logits_last) CK(m.stage.copy(logits_last, bs.logits.p, (size_t)B * V * sizeof(float), g_stream));
     TRY(sync_stream());
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));

@@ -229,7 +229,7 @@ template <int DKP> constexpr size_t delta_prepare_smem_bytes() { return sizeof(f
 // grid (chunks, heads).  DKP: key channels padded with zeros (64 or 128).
 template <int DKP>
 __global__ void __launch_bounds__(256) delta_chunk_prepare_kernel(DeltaChunkArgs c, StepMeta m) {
-    pdl_launch_dependents();
+    // (no early start for the walk behind this: its few long blocks would crowd on the SMs that empty first)
     pdl_wait_prior_grid();
     constexpr int C = kDeltaChunk, LDK = DKP + 4, LDV = 132;
     extern __shared__ __align__(16) float dsm[];

@@ -16,7 +16,9 @@
 #include <string>
 #include <vector>
 
+#include "stage_out.cuh"
 #include "seq_kernels.cuh"
+#include "seq_wkv.cuh"
 #include "seq_gemm_tc.cuh"
 #include "seq_attn_tc.cuh"
 #include "seq_recurrent.cuh"
@@ -266,6 +268,7 @@ struct Model {
     int max_aux = 0, max_aux2 = 0, max_route = 0;
     bool any_rgbuf = false;
     DevBuf<int> meta, picks;
+    DevBuf<float> wkv_M;         // chunked recurrence: products inside the chunks of 16 tokens, then the chunks' decays
     DevBuf<uint8_t> kv_images;   // split keys and values of the portions' attention (one layer run's, rewritten by the next)
     DevBuf<__nv_bfloat16> abf;   // bf16 copy of a product's activations for the tcgen05 path: [rows][max_k]
     DevBuf<int> attn_arrived;    // split-key attention: finished splits of a (row, head), zero between launches
@@ -280,6 +283,7 @@ struct Model {
     int max_heads_v = 0;         // max over attention layers of heads * (vdim + 2)
     DevBuf<int> err;             // device flag: a bounded wait in a kernel ran out
     int max_k = 0;
+    StageOut stage;
     int* meta_host = nullptr;
     size_t meta_host_cap = 0;
     int max_proj = 0, max_att = 0, max_ff = 0, max_rank = 0;
@@ -1067,7 +1071,7 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
         if (m.meta_host) cudaFreeHost(m.meta_host);
         m.meta_host = nullptr;
         m.meta_host_cap = 0;
-        CK(cudaMallocHost(&m.meta_host, n_meta * 2 * sizeof(int)));
+        CK(cudaMallocHost(&m.meta_host, (n_meta * 2 + 1) * sizeof(int)));   // (+ the error flag)
         m.meta_host_cap = n_meta * 2;
     }
     TRY(m.meta.ensure(m.meta_host_cap));
@@ -1753,7 +1757,16 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
             a.w0 = L.w0; a.u = L.u;
             a.state = R.state.p; a.out = m.att.p; a.heads = L.d.heads; a.dim = d;
             const dim3 grid(E, L.d.heads);
-            if (d == 32) TRY(launch_dep(wkv_scan_split_kernel<32, 8, 4>, dim3(E, L.d.heads, 1), dim3(128), 0, a, sm));
+            int longest = 0, chunks = 0;
+            for (int e = 0; e < E; ++e) { longest = std::max(longest, counts[e]); chunks += (counts[e] + kWkvChunk - 1) / kWkvChunk; }
+            if (longest >= kWkvChunkedMinRows && (d == 32 || d == 64 || d == 128) && m.wkv_M.ensure((size_t)chunks * L.d.heads * (kWkvChunk * kWkvChunk + d)) == 0) {
+                WkvChunkArgs ca{a, m.wkv_M.p, m.wkv_M.p + (size_t)chunks * L.d.heads * kWkvChunk * kWkvChunk};
+                const dim3 pg(chunks, L.d.heads), sg(E, L.d.heads, d / kWkvCols);
+                if (d == 32) { TRY(launch_dep(wkv_chunk_prepare_kernel<32>, pg, dim3(128), 0, ca, sm)); TRY(launch_dep(wkv_chunk_scan_kernel<32>, sg, dim3(128), wkv_chunk_smem_bytes(32), ca, sm)); }
+                else if (d == 64) { TRY(launch_dep(wkv_chunk_prepare_kernel<64>, pg, dim3(256), 0, ca, sm)); TRY(launch_dep(wkv_chunk_scan_kernel<64>, sg, dim3(256), wkv_chunk_smem_bytes(64), ca, sm)); }
+                else { TRY(launch_dep(wkv_chunk_prepare_kernel<128>, pg, dim3(512), 0, ca, sm)); TRY(launch_dep(wkv_chunk_scan_kernel<128>, sg, dim3(512), wkv_chunk_smem_bytes(128), ca, sm)); }
+                LAUNCHED();
+            } else if (d == 32) TRY(launch_dep(wkv_scan_split_kernel<32, 8, 4>, dim3(E, L.d.heads, 1), dim3(128), 0, a, sm));
             else if (d == 64) TRY(launch_dep(wkv_scan_split_kernel<64, 8, 8>, dim3(E, L.d.heads, 2), dim3(256), 0, a, sm));
             else if (d == 128) TRY(launch_dep(wkv_scan_split_kernel<128, 4, 16>, dim3(E, L.d.heads, 4), dim3(512), 0, a, sm));
             else {
@@ -1931,12 +1944,13 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     if (smp.on) {
         CK(cudaMemcpyAsync(smp.out_tokens, m.picks.p, (size_t)E * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
         if (smp.out_logprobs) CK(cudaMemcpyAsync(smp.out_logprobs, m.logprobs.p, (size_t)E * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
-    } else if (n_want > 0 && logits_host) {
-        CK(cudaMemcpyAsync(logits_host, m.logits.p, (size_t)n_want * V * sizeof(float), cudaMemcpyDeviceToHost, g_stream));
     }
-    int kerr = 0;
-    CK(cudaMemcpyAsync(&kerr, m.err.p, sizeof(int), cudaMemcpyDeviceToHost, g_stream));
+    // (the flag goes to pinned memory behind the step's table: the copies in front of the logits must not wait for the stream)
+    int* kerr_host = m.meta_host + m.meta_host_cap;
+    CK(cudaMemcpyAsync(kerr_host, m.err.p, sizeof(int), cudaMemcpyDeviceToHost, g_stream));
+    if (!smp.on && n_want > 0 && logits_host) CK(m.stage.copy(logits_host, m.logits.p, (size_t)n_want * V * sizeof(float), g_stream));
     CK(cudaStreamSynchronize(g_stream));
+    const int kerr = *kerr_host;
     if (kerr) return fail("step: a bounded wait inside a kernel ran out (tensor-core product pipeline)");
     CK(cudaEventElapsedTime(&m.last_ms, m.ev0, m.ev1));
     for (int e = 0; e < E; ++e) m.seqs[seqs[e]].len += counts[e];
@@ -2121,6 +2135,8 @@ int ti_seq_init(int device) {
     TI_LAT_ATTR(512, 512, 32, true);
     TI_LAT_ATTR(512, 512, 32, false);
 #undef TI_LAT_ATTR
+    CK(cudaFuncSetAttribute(wkv_chunk_scan_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wkv_chunk_smem_bytes(64)));
+    CK(cudaFuncSetAttribute(wkv_chunk_scan_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wkv_chunk_smem_bytes(128)));
     CK(cudaFuncSetAttribute(delta_chunk_prepare_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)delta_prepare_smem_bytes<64>()));
     CK(cudaFuncSetAttribute(delta_chunk_prepare_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)delta_prepare_smem_bytes<128>()));
     CK(cudaFuncSetAttribute(delta_chunk_scan_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)delta_chunk_smem_bytes<64>()));
@@ -2631,6 +2647,7 @@ int ti_seq_model_finalize(ti_seq_model_t h) {
     m.max_k = std::max({m.max_k, 2 * D, m.max_att, m.max_ff, m.max_rank, D});
     TRY(m.err.alloc(1));
     CK(cudaMemset(m.err.p, 0, sizeof(int)));
+    if (m.stage.open() != cudaSuccess) cudaGetLastError();   // (logits then take the driver's own way)
     CK(cudaEventCreate(&m.ev0));
     CK(cudaEventCreate(&m.ev1));
     m.finalized = true;
