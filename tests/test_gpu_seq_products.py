@@ -69,3 +69,20 @@ def test_recurrence_in_chunks_equals_tokens(dim, first, rows):
     # fp32 throughout; sums of up to 16 tokens and 128 channels in another order
     for want, g in ((binusun_plain.forward(cfg, W, toks), np.concatenate(got)), (binusun_plain.forward(cfg, W, other), both[:17])):
         assert np.abs(g - want).max() <= 2e-4 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("rows", [33, 130])
+@pytest.mark.parametrize("width,rank,ff", [(72, 64, 72), (136, 72, 200), (264, 64, 1032), (136, 32, 200), (68, 64, 68)])   # the last two: mixes in fp32
+def test_mixes_and_gated_rows_in_bf16(rows, width, rank, ff):
+    """Token-shift mixes and gated feed-forward rows that go to their products as bf16, for rows behind an earlier portion and of two requests."""
+    cfg = binusun_cases.make_config([binusun_cases.wkv_layer(heads=2, dim=40, rank=rank, ff=ff)], width=width)
+    W = binusun_cases.random_weights(cfg, seed=rows + ff, decay_bias=-2.0)
+    rng = np.random.default_rng(rows)
+    toks, other = [[int(t) for t in rng.integers(0, cfg["vocab"], n)] for n in (20 + rows, 35)]
+    m = binusun_cases.build_engine(cfg, W, "bfloat16")
+    s, o = m.open(), m.open()
+    head = m.step([(s, toks[:20])], [range(20)])
+    both = m.step([(o, other), (s, toks[20:])], [range(35), range(rows)])
+    m.free()
+    for want, got in ((binusun_plain.forward(cfg, W, toks), np.concatenate([head, both[35:]])), (binusun_plain.forward(cfg, W, other), both[:35])):
+        assert np.abs(got - want).max() <= TOL * np.abs(want).max()

@@ -43,8 +43,8 @@ __global__ void rope_kv_batch_kernel(float* qkv, int H, int rope_dim, const floa
 // interleaved (gate_i, up_i) columns of gu[M][2K] (SwiGLU fused in front of the down projection, :918, :1729).  Same expressions as
 // rmsnorm_digits_kernel (prefill.cuh).
 // Threads (digits_threads): few rows are a matter of latency, 1024 threads a row; from a row per SM on the rows are a matter of bandwidth, and a thread
-// takes its full sixteen values so that several rows share an SM (2047 rows of 4096 behind a norm, us: 52 with 1024 threads a row, 20 with 256; 332 rows of
-// 2048: 12 and 7).
+// takes its full sixteen values so that several rows share an SM (mean of a layer's four conversions, us, with 1024 threads a row and so: 2048 rows of
+// 4096 and 11008: 54 and 34.5; 333 rows of 2048 and 5632: 11.5 and 7.0).
 constexpr int kDigitsThreads = 1024, kDigitsVecs = 4;   // most threads a row; 4 float4 per thread
 inline int digits_threads(int rows, int k_pad, int sms) {
     return rows <= sms ? kDigitsThreads : std::min(kDigitsThreads, std::max(128, ((k_pad + 4 * kDigitsVecs - 1) / (4 * kDigitsVecs) + 31) / 32 * 32));

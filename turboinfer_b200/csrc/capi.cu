@@ -1237,8 +1237,9 @@ int pf_digits(Model& m, const float* x, const float* norm_w, int M, int K, int m
 }
 
 // Prompts run on the tensor-core GEMMs from a few tokens on: one pass over the layers costs about three steps of the decode engine (four
-// 7B-wide layers, us: 16 tokens at once 330, one at a time 16 x 134).  The GEMMs read a byte copy of the weights, made on first use; below the 33 tokens from which
-// the copy has always been made it must leave room on the GPU.
+// layers of 2048, kernel time in us: 16 tokens at once 410, one at a time 16 x 134), so that from six tokens on it is ahead with some margin.
+// The GEMMs read a byte copy of the weights, made on first use; below the 33 tokens from which the copy has always been made it must leave
+// room on the GPU.
 constexpr int kPromptGemmTokens = 6;
 bool kmajor_fits(const Model& m) {
     size_t need = 0;
@@ -1262,17 +1263,18 @@ bool prefill_gemm_eligible(const Model& m, int M) {
 struct PrefillRows { const int* tokens; int n_seq, P; const int* tables; int pages_per_seq; };
 
 // causal attention of the rows on tcgen05: the heads' keys and values are split into tile images, as many heads at a time as the image
-// buffer takes (a buffer that cannot be had is asked for in halves, down to one head)
+// buffer takes (a buffer that cannot be had is asked for in halves, down to one head; *done stays false when there is no room for that either)
 template <int DH>
-int prefill_attention(Model& m, const float* k_pool, const float* v_pool, const PrefillRows& pr, float scale) {
+int prefill_attention(Model& m, const float* k_pool, const float* v_pool, const PrefillRows& pr, float scale, bool* done) {
     const int H = m.cfg.hidden, heads = m.attn_heads, kt = (pr.P + kAtKT - 1) / kAtKT, tiles = pr.n_seq * kt;
     int per = at_heads_per_launch(heads, tiles, DH, DH, kAtImageBudget);
     while (m.pf_images.n < (size_t)per * tiles * at_record_bytes(DH, DH)) {
         if (m.pf_images.alloc((size_t)per * tiles * at_record_bytes(DH, DH)) == 0) break;
         cudaGetLastError();
-        if (per == 1) return 1;
+        if (per == 1) return 0;
         per = (per + 1) / 2;
     }
+    *done = true;
     for (int h0 = 0; h0 < heads; h0 += per) {
         const int nh = std::min(per, heads - h0);
         const PrefillKeys keys{k_pool, v_pool, pr.tables, pr.pages_per_seq, m.page_tokens, H, DH, DH, pr.P, kt, h0};
@@ -1308,19 +1310,18 @@ int prefill_gemm(Model& m, const PrefillRows& pr, Pool pool) {
         static const std::string attn_sel = getenv("TURBOINFER_B200_PREFILL_ATTN") ? getenv("TURBOINFER_B200_PREFILL_ATTN") : "";   // A/B: fp32 | tf32
         const bool attn_fp32 = attn_sel == "fp32", attn_tf32 = attn_sel == "tf32";
         const float att_scale = 1.0f / sqrtf((float)m.attn_dim);
-        if (!attn_fp32 && !attn_tf32 && m.attn_dim == 128) {          // tcgen05, split FP16 (attn_tc.cuh)
-            TRY(prefill_attention<128>(m, k_pool, v_pool, pr, att_scale));
-        } else if (!attn_fp32 && !attn_tf32 && m.attn_dim == 64) {
-            TRY(prefill_attention<64>(m, k_pool, v_pool, pr, att_scale));
-        } else {
+        bool done = false;   // tcgen05, split FP16 (attn_tc.cuh)
+        if (!attn_fp32 && !attn_tf32 && m.attn_dim == 128) TRY(prefill_attention<128>(m, k_pool, v_pool, pr, att_scale, &done));
+        if (!attn_fp32 && !attn_tf32 && m.attn_dim == 64) TRY(prefill_attention<64>(m, k_pool, v_pool, pr, att_scale, &done));
+        if (!done) {
             for (int i = 0; i < pr.n_seq; ++i) {   // sequence by sequence
                 float* q = m.pf_qkv.p + (size_t)i * pr.P * 3 * H;
                 float* out = m.pf_attn.p + (size_t)i * pr.P * H;
                 const int* table = pr.tables + (size_t)i * pr.pages_per_seq;
                 const dim3 tc_grid(m.attn_heads, (pr.P + kTcQ - 1) / kTcQ);
-                if (!attn_fp32 && m.attn_dim == 128)   // split TF32
+                if (attn_tf32 && m.attn_dim == 128)   // split TF32
                     causal_attention_tc_kernel<128><<<tc_grid, kTcThreads, attn_tc_smem_bytes<128>(), g_stream>>>(q, pr.P, H, att_scale, 0, k_pool, v_pool, table, m.page_tokens, out);
-                else if (!attn_fp32 && m.attn_dim == 64)
+                else if (attn_tf32 && m.attn_dim == 64)
                     causal_attention_tc_kernel<64><<<tc_grid, kTcThreads, attn_tc_smem_bytes<64>(), g_stream>>>(q, pr.P, H, att_scale, 0, k_pool, v_pool, table, m.page_tokens, out);
                 else
                     causal_attention_kernel<<<dim3(m.attn_heads, (pr.P + kPfQ - 1) / kPfQ), kPfThreads, kPfSmemBytes, g_stream>>>(q, pr.P, H, m.attn_dim, att_scale, 0, k_pool, v_pool,

@@ -102,8 +102,8 @@ TIB_HD size_t wtile_offset(int n, int k, int k_pad) {
     return ((size_t)(n / kGemmBN) * (k_pad / kGemmBK) + k / kGemmBK) * kGemmTileBytes + sw128_offset(n % kGemmBN, k % kGemmBK);
 }
 // packed streaming layout -> tile-major bytes, grid (slabs, parts), thread mapping of unpack_kernel.  A word of the packed layout is four
-// consecutive k of one column (INT8), or two such fours 32 k apart (INT4, low and high nibbles): whole words are stored (byte stores took four times as
-// long: 16 ms instead of 3 for 0.8 GB of INT8 weights, the first prompt of a model)
+// consecutive k of one column (INT8), or two such fours 32 k apart (INT4, low and high nibbles): whole words are stored (with byte stores the
+// first prompt of a model behind 0.8 GB of INT8 weights took 16 ms longer than the next one, now 7)
 __global__ void unpack_kmajor_kernel(const uint8_t* packed, QLayout L, int k_pad, uint8_t* wk) {
     const Slab slab = make_slab(L, blockIdx.x);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -425,8 +425,8 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 //     leaves the counter zeroed for the next GEMM;
 //   * two accumulators: the epilogue of a tile runs under the k-steps of the next.
 // warps 0..7: epilogue (warp w: weight columns 32 (w % 4) .., rows 16 (w / 4) ..), warp 8: TMEM allocation + MMA issue, warp 9: producer.
-// Measured (INT4 weights, 32 rows, us a launch in a chain of launches on a B200; before: whole column tiles, K split into at most eight):
-// see small_gemm_ctas() for the rule.
+// Measured (4096 x 22016, 32 rows, us a launch in a chain of launches on a B200): 31 with whole column tiles and K split into at most eight,
+// 22 now; the four products of a 4096-wide layer on average 29 -> 20.7, against 3 to 14 for their weight bytes.
 constexpr int kSmallRows = 32, kSmallEpiWarps = 8, kSmallThreads = 64 + 32 * kSmallEpiWarps;
 constexpr int kSmallRing = 196 * 1024;
 constexpr int kSmallTmemCols = 256;                                          // two accumulators of up to 96 columns
@@ -449,7 +449,8 @@ struct SmallArgs {
 };
 // first unit of CTA c (units * CTAs fits 32 bits: at most 2^22 units on 148 SMs)
 TIB_HD int small_unit(int units, int c, int ctas) { return (int)((uint32_t)units * (uint32_t)c / (uint32_t)ctas); }
-// CTAs of a launch: all SMs as long as each has at least `min_steps` k-steps (below that the fix-up of shared tiles costs more than it gives)
+// CTAs of a launch: all SMs as long as each has at least four k-steps, a
+// shorter run would be mostly the fix-up of its shared tiles.  Chosen, not swept: only matrices below 592 units (9.7 M weights) are concerned
 inline int small_gemm_ctas(int units, int sms) { return std::max(1, std::min(sms, units / 4)); }
 
 template <int R>

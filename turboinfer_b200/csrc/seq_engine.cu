@@ -1247,17 +1247,22 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     if (front) TRY(hyper(0, -1));
     // paged softmax attention of all rows of the step (prompt portions in tiles, the other rows one by one or split over their keys)
     auto h3_size = [](const AttnShape& s) { return s.dim <= 128 && s.vdim <= 128 && s.dim % 4 == 0 && s.vdim % 4 == 0 && s.v_ld == 0; };
-    auto h3_attention = [&](const StepMeta& sm, const AttnShape& s, const float* q, const float* kp, const float* vp, float* out) -> int {   // the portions' tiles
-        const int dk = at_pad(s.dim), dv = at_pad(s.vdim), group = s.heads / s.kv_heads;
-        // keys and values are split into tile images first, as many heads at a time as the image buffer takes (a buffer that cannot be had
-        // is asked for in halves, down to one head)
+    // keys and values are split into tile images first: as many heads at a time as the image buffer takes (a buffer that cannot be had is
+    // asked for in halves, down to one head; 0: no room for one either)
+    auto h3_heads = [&](const AttnShape& s) {
+        const int dk = at_pad(s.dim), dv = at_pad(s.vdim);
         int per = at_heads_per_launch(s.kv_heads, n_ktiles, dk, dv, kAtImageBudget);
         while (m.kv_images.n < (size_t)per * n_ktiles * at_record_bytes(dk, dv)) {
             if (m.kv_images.alloc((size_t)per * n_ktiles * at_record_bytes(dk, dv)) == 0) break;
             cudaGetLastError();
-            if (per == 1) return 1;
+            if (per == 1) return 0;
             per = (per + 1) / 2;
         }
+        return per;
+    };
+    auto h3_attention = [&](const StepMeta& sm, const AttnShape& s, const float* q, const float* kp, const float* vp, float* out) -> int {   // the portions' tiles
+        const int dk = at_pad(s.dim), dv = at_pad(s.vdim), group = s.heads / s.kv_heads, per = h3_heads(s);
+        if (per == 0) return 1;
         for (int g0 = 0; g0 < s.kv_heads; g0 += per) {
             const int ng = std::min(per, s.kv_heads - g0);
             const SeqKeys keys{sm, s, d_ktiles, kp, vp, s.dim, s.vdim, g0};
@@ -1284,7 +1289,7 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
         const size_t tsmem = attn_tiled_smem_bytes(s.dim, s.vdim, v_in_k);
         const bool tiled_ok = g_use_tiled_attn && n_tiles > 0 && s.dim % 4 == 0 && s.vdim % 4 == 0 && s.vdim <= 512 && tsmem <= g_smem_optin && (s.v_ld % 4 == 0);
         // bf16 mode, head sizes up to 128 in fours: the split-half tensor-core kernel (fp32-accurate); fp32 mode keeps true fp32 arithmetic
-        const bool h3_ok = g_use_tiled_attn && g_use_tc && bf && n_tiles128 > 0 && h3_size(s);
+        const bool h3_ok = g_use_tiled_attn && g_use_tc && bf && n_tiles128 > 0 && h3_size(s) && !only_small && h3_heads(s) > 0;
         // bf16 mode, a shared key/value head with the values inside the key rows (latent attention), instantiated sizes: tensor cores
         const bool lat_size = (s.dim == 320 && s.vdim == 256) || (s.dim == 192 && s.vdim == 128) || (s.dim == 160 && s.vdim == 128) || (s.dim == s.vdim && s.dim % 4 == 0 && s.dim <= 512);
         const bool lat_ok = g_use_tiled_attn && g_use_tc && bf && n_tiles > 0 && v_in_k && (!s.out_gate || s.gate) && !s.qk_norm && lat_size;
@@ -1488,7 +1493,7 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
         x.kv_heads = H; x.dim = d.dim; x.vdim = d.vdim; x.v_ld = 0; x.ld = nf; x.out_ld = ldo; x.egate = eg; x.egate_ld = nf;
         const size_t xrows = xpages.size() * kPageTokens;
         const double direct = xpairs * 6.0 * (d.dim + d.vdim) + 0.4 * (double)xrows * rank * (d.dim + d.vdim);   // (0.4: two operations on tcgen05, a fifth of the time)
-        if (L.uk && xrows > 32 && g_use_tiled_attn && h3_size(x) && direct < xpairs * 12.0 * rank && (double)xrows * H * (d.dim + d.vdim) * 4 < 4e9) {
+        if (L.uk && xrows > 32 && g_use_tiled_attn && h3_size(x) && direct < xpairs * 12.0 * rank && (double)xrows * H * (d.dim + d.vdim) * 4 < 4e9 && h3_heads(x) > 0) {
             TRY(m.cx.ensure(xrows * rank));
             TRY(m.kx.ensure(xrows * H * d.dim));
             TRY(m.vx.ensure(xrows * H * d.vdim));
@@ -1741,15 +1746,22 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
                 TRY(launch_dep(wkv_save_prev_kernel, dim3(E), dim3(nt), 0, m.h.p, sm, D, R.prev.p));
                 LAUNCHED();
             } else {
-                TRY(launch_dep(wkv_mix_kernel, dim3(T), dim3(nt), 0, m.h.p, sm, D, L.mu.p, R.prev.p, m.mixes.p));
+                // the mixes go out as bf16 when all five products take bf16 rows (tc_ok also says D % 8 == 0), as fp32 when any of them does not
+                const bool mix16 = tc_ok(m, L.r, T, C, D) && tc_ok(m, L.k, T, C, D) && tc_ok(m, L.v, T, C, D) && tc_ok(m, L.g, T, C, D) && tc_ok(m, L.w1, T, rank, D);
+                __nv_bfloat16* mix = reinterpret_cast<__nv_bfloat16*>(m.mixes.p);
+                if (mix16) TRY(launch_dep(wkv_mix_bf16_kernel, dim3(T), dim3(256), 0, m.h.p, sm, D, L.mu.p, R.prev.p, mix));
+                else TRY(launch_dep(wkv_mix_kernel, dim3(T), dim3(nt), 0, m.h.p, sm, D, L.mu.p, R.prev.p, m.mixes.p));
                 LAUNCHED();
                 TRY(launch_dep(wkv_save_prev_kernel, dim3(E), dim3(nt), 0, m.h.p, sm, D, R.prev.p));
                 LAUNCHED();
-                TRY(gemm(m, m.mixes.p + 0 * TD, D, L.r, pr, C, T, C, D));
-                TRY(gemm(m, m.mixes.p + 1 * TD, D, L.k, pk, C, T, C, D));
-                TRY(gemm(m, m.mixes.p + 2 * TD, D, L.v, pv, C, T, C, D));
-                TRY(gemm(m, m.mixes.p + 3 * TD, D, L.g, pg, C, T, C, D, EPI_SILU));
-                TRY(gemm(m, m.mixes.p + 4 * TD, D, L.w1, m.lora.p, rank, T, rank, D, EPI_TANH));
+                auto product = [&](int s, const void* W, float* out, int n, int epi) {
+                    return mix16 ? gemm_tc(m, mix + s * TD, D, W, out, n, T, n, D, epi) : gemm(m, m.mixes.p + s * TD, D, W, out, n, T, n, D, epi);
+                };
+                TRY(product(0, L.r, pr, C, EPI_NONE));
+                TRY(product(1, L.k, pk, C, EPI_NONE));
+                TRY(product(2, L.v, pv, C, EPI_NONE));
+                TRY(product(3, L.g, pg, C, EPI_SILU));
+                TRY(product(4, L.w1, m.lora.p, rank, EPI_TANH));
             }
             TRY(gemm(m, m.lora.p, rank, L.w2, pz, C, T, C, rank));
             WkvArgs a{};
@@ -1845,7 +1857,14 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
                     TRY(gemm(m, ff_in, D, L.gateup, m.act.p, F, T, F, D, EPI_NONE, 1.f, &f));
                 } else {
                     TRY(gemm(m, ff_in, D, L.gateup, m.proj.p, 2 * F, T, 2 * F, D));
-                    TRY(glu(m.proj.p, 2 * F, F, L, m.act.p, F));
+                    if (tc_ok(m, L.down, T, D, F) && m.abf.p && (size_t)T * F <= m.abf.n) {   // the down product's rows as bf16 straight away
+                        TRY(launch_dep(glu_kernel<4, __nv_bfloat16>, dim3(grid_for((size_t)T * F / 4)), dim3(256), 0, m.proj.p, 2 * F, F, L.d.ff_act, L.d.ff_limit, m.abf.p, F, T));
+                        LAUNCHED();
+                        TRY(gemm_tc(m, m.abf.p, F, L.down, m.mo.p, D, T, D, F));
+                        down_done = true;
+                    } else {
+                        TRY(glu(m.proj.p, 2 * F, F, L, m.act.p, F));
+                    }
                 }
             } else if (L.d.ff_kind == TI_SEQ_FF_POLYNORM) {
                 TRY(gemm(m, m.h.p, D, L.ffront, m.proj.p, L.n_ffront, T, L.n_ffront, D));

@@ -267,7 +267,7 @@ __device__ __forceinline__ float mix_cap(float v, const AttnShape& s) {
 __device__ __forceinline__ size_t mix_token(const int* table, int j) { return (size_t)table[j / kPageTokens] * kPageTokens + j % kPageTokens; }
 
 // pass 1, prompt portions: grid (groups of the band's 64-key tiles, tiles of the batch, heads).  TC (bf16 mode, head size in whole 16-element
-// steps): the product runs on the warp-level tensor cores at fp32 accuracy, the split-half scheme of window_attention_h3_kernel --
+// steps): the product runs on the warp-level tensor cores at fp32 accuracy, the split-half scheme of attn_tc.cuh --
 // every fp32 operand is split into two fp16 halves (x = hi + lo) as it is staged, and lo*hi + hi*lo + hi*hi is accumulated in fp32
 // by mma.sync m16n8k16; a warp owns 16 rows x 32 keys.  Otherwise true fp32 multiply-adds, 4 rows x 4 keys a thread.
 template <bool TC>

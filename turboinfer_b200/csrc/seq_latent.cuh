@@ -96,7 +96,7 @@ __global__ void latent_gather_kernel(const float* pool, int ld, int rank, const 
 }
 
 // Prompt portions of latent attention on the warp-level tensor cores at fp32 accuracy (bf16 mode): the split-half scheme of
-// window_attention_h3_kernel (x = hi + lo with two fp16 halves, hi*hi + hi*lo + lo*hi accumulated in fp32 by mma.sync m16n8k16;
+// attn_tc.cuh (x = hi + lo with two fp16 halves, hi*hi + hi*lo + lo*hi accumulated in fp32 by mma.sync m16n8k16;
 // scores, softmax with the sink and running sums in fp32) for ONE shared key/value head whose values are the leading DV
 // coordinates of its DK-wide key rows -- so the key tile in shared memory is also the value tile and nothing is loaded twice.
 // A block owns up to 64 consecutive rows of one sequence and one query head; its 8 warps are 4 row groups x 2 halves of the
