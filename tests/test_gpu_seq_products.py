@@ -86,3 +86,16 @@ def test_mixes_and_gated_rows_in_bf16(rows, width, rank, ff):
     m.free()
     for want, got in ((binusun_plain.forward(cfg, W, toks), np.concatenate([head, both[35:]])), (binusun_plain.forward(cfg, W, other), both[:35])):
         assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+
+
+@pytest.mark.parametrize("rows", [1, 3, 8])
+@pytest.mark.parametrize("width,ff,vocab", [(256, 4736, 4753), (256, 9488, 14209), (288, 2400, 9473)])   # 16 columns x 296 blocks = 4736: one, two, three turns a block
+def test_few_rows_with_several_column_tiles_a_block(rows, width, ff, vocab):
+    cfg = binusun_cases.make_config([binusun_cases.attn_layer(heads=3, kv_heads=1, dim=40, vdim=24, rot_dims=8, window=50, ff=ff)], vocab=vocab, width=width)
+    W = binusun_cases.random_weights(cfg, seed=rows)
+    toks = [int(t) for t in np.random.default_rng(rows).integers(0, vocab, rows)]
+    m = binusun_cases.build_engine(cfg, W, "bfloat16")
+    got = one_step(m, toks)
+    m.free()
+    want = binusun_plain.forward(cfg, W, toks)
+    assert np.abs(got - want).max() <= TOL * np.abs(want).max()
