@@ -1,0 +1,34 @@
+"""A token whose values are not finite touches the rows that see it, not the ones in front of it."""
+import numpy as np
+import pytest
+
+import binusun_cases
+import binusun_plain
+
+pytestmark = pytest.mark.gpu
+
+# rows of bf16 products (2^-9 of a value), a dozen roundings; fp32 sums in another order otherwise
+TOL = {"bfloat16": 12 * 2.0 ** -9, "float32": 2e-4}
+
+
+def rows_in_front(cfg, dtype, n, at, value):
+    """The first `at` rows of a portion of n tokens whose token number `at` has an embedding of `value`, and what they ought to be."""
+    W = binusun_cases.random_weights(cfg, seed=n + at, decay_bias=-2.0)
+    bad = cfg["vocab"] - 1
+    toks = [int(t) for t in np.random.default_rng(at).integers(0, bad, n)]
+    toks[at] = bad
+    want = binusun_plain.forward(cfg, W, toks[:at])
+    W["embed"][bad] = value
+    m = binusun_cases.build_engine(cfg, W, dtype)
+    s = m.open()
+    got = m.step([(s, toks)], [range(n)])
+    m.free()
+    return got[:at], want
+
+
+@pytest.mark.parametrize("dim", [32, 64, 128])
+@pytest.mark.parametrize("at,value", [(37, np.inf), (63, np.nan), (65, -np.inf)])   # inside, at the end and at the beginning of a chunk of 16
+def test_recurrence_in_chunks_is_causal(dim, at, value):
+    cfg = binusun_cases.make_config([binusun_cases.wkv_layer(heads=2, dim=dim, rank=8)], width=64)
+    got, want = rows_in_front(cfg, "float32", 90, at, value)
+    assert np.abs(got - want).max() <= TOL["float32"] * np.abs(want).max()

@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(4 * D) wkv_chunk_scan_kernel(WkvChunkArgs a, S
 #pragma unroll
                 for (int i = 0; i < NW; ++i) s4[i & 3] += part[(i * L + t) * kWkvCols + col];
 #pragma unroll
-                for (int i = 0; i < L; ++i) s4[i & 3] = fmaf(M[t * L + i], v[i * kWkvCols + col], s4[i & 3]);   // (zero behind t)
+                for (int i = 0; i < L; ++i) s4[i & 3] = fmaf(M[t * L + i], i <= t ? v[i * kWkvCols + col] : 0.f, s4[i & 3]);   // (M is zero behind t, but a later token's v may be infinite)
                 a.w.out[(size_t)(t0 + q * L + t) * C + (size_t)hd * D + col0 + col] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
             }
         }
