@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
     } else {
         reg_alloc<208>();
         const int q = warp & 3, r = q * 32 + lane;
+        const int qp = r < M ? pos0 + r : -1, lo = r < M ? s.first_key(pos0 + r) : 0;
         float o[DV];
 #pragma unroll
         for (int c = 0; c < DV; ++c) o[c] = 0.f;
@@ -338,12 +339,17 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
             if (!ok) break;
             tc_fence_after();
             const float f = factor[slot * kAtQ + r];
+            // (a tile without a key the row sees is left out, not added as zeros: its values may be infinite, and zero times infinity is not zero)
+            const int t0 = (first + i) * kAtKT;
+            const bool seen = t0 <= qp && t0 + kAtKT > lo;
 #pragma unroll
             for (int c = 0; c < DV; c += 32) {
                 uint32_t v[32];
                 tmem_ld32(v, tmem + ((uint32_t)(q * 32) << 16) + kOCol + b * DV + c);
+                if (seen) {
 #pragma unroll
-                for (int e = 0; e < 32; ++e) o[c + e] = fmaf(o[c + e], f, __uint_as_float(v[e]));
+                    for (int e = 0; e < 32; ++e) o[c + e] = fmaf(o[c + e], f, __uint_as_float(v[e]));
+                }
             }
             tc_fence_before();
             __syncwarp();
