@@ -1,0 +1,102 @@
+"""Calls on a GPU that has no room for their larger buffers, and what calls allocate at all.  A shim in front of the CUDA runtime's allocation
+functions (preloaded into a child process) refuses requests above a size, the device ones with the runtime's own out-of-memory error, and keeps
+count."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+static size_t device_limit = ~(size_t)0, pinned_limit = ~(size_t)0;
+static long n_refused, n_pinned, total;
+static size_t largest;
+void shim_limits(size_t device, size_t pinned) { device_limit = device; pinned_limit = pinned; n_refused = n_pinned = 0; total = 0; largest = 0; }
+long shim_refused(void) { return n_refused; }
+long shim_pinned(void) { return n_pinned; }
+long shim_total(void) { return total; }
+long shim_largest(void) { return (long)largest; }
+static void* real(const char* name) { return dlsym(dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), name); }
+int cudaMalloc(void** p, size_t n) {
+    int (*f)(void**, size_t) = (int (*)(void**, size_t))real("cudaMalloc");
+    if (n > device_limit) { ++n_refused; return f(p, (size_t)1 << 50); }
+    total += (long)n;
+    if (n > largest) largest = n;
+    return f(p, n);
+}
+int cudaHostAlloc(void** p, size_t n, unsigned int flags) {
+    int (*f)(void**, size_t, unsigned int) = (int (*)(void**, size_t, unsigned int))real("cudaHostAlloc");
+    ++n_pinned;
+    if (n > pinned_limit) { ++n_refused; return 2; }
+    return f(p, n, flags);
+}
+"""
+
+COMMON = r"""
+import ctypes, os, sys
+sys.path[:0] = [ROOT, os.path.join(ROOT, "tests")]
+import numpy as np
+shim = ctypes.CDLL(None)
+NONE = 2 ** 63
+def limits(device=NONE, pinned=NONE): shim.shim_limits(ctypes.c_size_t(device), ctypes.c_size_t(pinned))
+for f in ("refused", "pinned", "total", "largest"): getattr(shim, "shim_" + f).restype = ctypes.c_long
+import binusun_cases, binusun_plain
+import turboinfer_b200 as tb
+from helpers import make_model, prompt_tokens
+TOL16 = 12 * 2.0 ** -9   # a dozen roundings to bf16
+
+META = dict(vocab=160, hidden=256, layers=2, heads=4, inter=1024)
+def llama(**kw): return tb.Model(META, tb.Q_INT8, attn_mode=1, rope_mode=1, max_seq=160).load(make_model(META, norm_jitter=0.1))
+def prompts(n, batch=4): return np.array([prompt_tokens(n, META["vocab"], offset=3 * b) for b in range(batch)], dtype=np.int32)
+def alone(n, new):   # the same answers, a request at a time through the decode engine
+    os.environ["TURBOINFER_B200_PREFILL"] = "decode"
+    m = llama()
+    out = np.array([m.generate_greedy(list(p), new)[0] for p in prompts(n)])
+    m.free()
+    del os.environ["TURBOINFER_B200_PREFILL"]
+    return out
+def seq(layers, dtype, **kw):
+    cfg = binusun_cases.make_config(layers, width=64)
+    W = binusun_cases.random_weights(cfg, seed=7, decay_bias=-2.0)
+    return cfg, W, binusun_cases.build_engine(cfg, W, dtype, **kw)
+def tokens(n, seed=1): return [int(t) for t in np.random.default_rng(seed).integers(0, 97, n)]
+def close(got, want, tol): assert np.abs(got - want).max() <= tol * np.abs(want).max(), np.abs(got - want).max() / np.abs(want).max()
+"""
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    d = tmp_path_factory.mktemp("shim")
+    src, lib = d / "shim.c", d / "shim.so"
+    src.write_text(SHIM)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", str(lib), str(src), "-ldl"], check=True)
+    return str(lib)
+
+
+def child(shim, code):
+    p = subprocess.run([sys.executable, "-c", "ROOT = %r\n" % ROOT + COMMON + code], env=dict(os.environ, LD_PRELOAD=shim), capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stdout[-2000:] + p.stderr[-3000:]
+
+
+def test_recurrence_without_room_for_chunks(shim):
+    # 96 rows both times, in 6 chunks of 16 tokens and then in 12: there is no room for the products inside the second step's chunks
+    child(shim, """
+cfg, W, m = seq([binusun_cases.wkv_layer(heads=2, dim=32, rank=8)], "float32", max_seqs=10)
+a = tokens(96)
+s = m.open()
+close(m.step([(s, a)], [range(96)]), binusun_plain.forward(cfg, W, a), 2e-4)
+m.close(s)
+parts = [tokens(64, 2)] + [tokens(4, 3 + i) for i in range(8)]
+ids = [m.open() for _ in parts]
+limits(device=20000)
+got = m.step(list(zip(ids, parts)), [range(len(p)) for p in parts])
+assert shim.shim_refused() > 0
+close(got, np.concatenate([binusun_plain.forward(cfg, W, p) for p in parts]), 2e-4)
+""")

@@ -105,7 +105,11 @@ struct DevBuf {
         release();
         if (count == 0) return 0;
         cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-        if (e != cudaSuccess) return fail("cudaMalloc(%zu bytes) failed: %s", count * sizeof(T), cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            cudaGetLastError();   // (reported here: the check behind the next launch, a fall-back's or another call's, must not see it again)
+            p = nullptr;
+            return fail("cudaMalloc(%zu bytes) failed: %s", count * sizeof(T), cudaGetErrorString(e));
+        }
         n = count;
         return 0;
     }
@@ -1270,7 +1274,6 @@ int prefill_attention(Model& m, const float* k_pool, const float* v_pool, const 
     int per = at_heads_per_launch(heads, tiles, DH, DH, kAtImageBudget);
     while (m.pf_images.n < (size_t)per * tiles * at_record_bytes(DH, DH)) {
         if (m.pf_images.alloc((size_t)per * tiles * at_record_bytes(DH, DH)) == 0) break;
-        cudaGetLastError();
         if (per == 1) return 0;
         per = (per + 1) / 2;
     }

@@ -94,7 +94,11 @@ struct DevBuf {
         release();
         if (count == 0) return 0;
         cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-        if (e != cudaSuccess) return fail("cudaMalloc(%zu bytes) failed: %s", count * sizeof(T), cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            cudaGetLastError();   // (reported here: the check behind the next launch, a fall-back's or another call's, must not see it again)
+            p = nullptr;
+            return fail("cudaMalloc(%zu bytes) failed: %s", count * sizeof(T), cudaGetErrorString(e));
+        }
         n = count;
         return 0;
     }
@@ -1254,7 +1258,6 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
         int per = at_heads_per_launch(s.kv_heads, n_ktiles, dk, dv, kAtImageBudget);
         while (m.kv_images.n < (size_t)per * n_ktiles * at_record_bytes(dk, dv)) {
             if (m.kv_images.alloc((size_t)per * n_ktiles * at_record_bytes(dk, dv)) == 0) break;
-            cudaGetLastError();
             if (per == 1) return 0;
             per = (per + 1) / 2;
         }
