@@ -100,3 +100,40 @@ got = m.step(list(zip(ids, parts)), [range(len(p)) for p in parts])
 assert shim.shim_refused() > 0
 close(got, np.concatenate([binusun_plain.forward(cfg, W, p) for p in parts]), 2e-4)
 """)
+
+
+def test_batch_after_one_without_room(shim):
+    # scratch that could not be made: the call fails, and nothing of it may be left for the next one -- neither for one of the same shape,
+    # whose captured steps hold the old addresses, nor for one with fewer rows
+    child(shim, """
+tb.init(0)
+want = alone(2, 5)
+m = llama()
+assert np.array_equal(m.generate_batch_greedy(prompts(2), 5)[0], want)
+limits(device=2000)
+try:
+    m.generate_batch_greedy(prompts(50), 5)
+    raise SystemExit("no error")
+except tb.B200Error:
+    pass
+limits()
+assert np.array_equal(m.generate_batch_greedy(prompts(2), 5)[0], want)
+assert np.array_equal(m.generate_batch_greedy(prompts(50), 5)[0], alone(50, 5))
+""")
+
+
+def test_first_batch_without_room(shim):
+    child(shim, """
+tb.init(0)
+want = alone(50, 5)
+m = llama()
+for room in (300000, 100000, 10000, 1000):   # the failure moves forward through what a batch allocates
+    limits(device=room)
+    try:
+        m.generate_batch_greedy(prompts(50), 5)
+        raise SystemExit("no error")
+    except tb.B200Error:
+        pass
+limits()
+assert np.array_equal(m.generate_batch_greedy(prompts(50), 5)[0], want)
+""")

@@ -1385,6 +1385,9 @@ int ensure_pf_scratch(Model& m, int M) {
         for (QWeight* w : {ly.qkv.get(), ly.o.get(), ly.gateup.get(), ly.down.get()}) upd(w);
     upd(m.lm_head.get());
     if (M > m.pf_cap || m.pf_planes.n < (size_t)3 * m_pad * kmax) {
+        // from the first of these on the old buffers are gone: unless all of them succeed there is no scratch, and captured steps are stale in any case
+        m.pf_cap = 0;
+        ++m.pf_gen;
         TRY(m.pf_x.alloc((size_t)M * H));
         TRY(m.pf_qkv.alloc((size_t)M * 3 * H));
         TRY(m.pf_attn.alloc((size_t)M * H));
@@ -1394,7 +1397,6 @@ int ensure_pf_scratch(Model& m, int M) {
         TRY(m.pf_sxf.alloc(M));
         TRY(m.pf_planes.alloc((size_t)3 * m_pad * kmax));
         m.pf_cap = M;
-        ++m.pf_gen;
     }
     size_t nmax = 0;
     auto updn = [&](QWeight* w) { if (w) nmax = std::max(nmax, (size_t)(4 * w->L.U + kGemmBN - 1) / kGemmBN * kGemmBN); };
@@ -1402,10 +1404,11 @@ int ensure_pf_scratch(Model& m, int M) {
         for (QWeight* w : {ly.qkv.get(), ly.o.get(), ly.gateup.get(), ly.down.get()}) updn(w);
     updn(m.lm_head.get());
     if (m.pf_cnt.n < nmax / kGemmBN) {
+        ++m.pf_gen;
+        m.pf_cnt.release();   // (the counters come last: while they are missing, so is the rest)
         TRY(m.pf_ws.alloc((size_t)2 * g_num_sms * kSmallRows * kGemmBN));
         TRY(m.pf_cnt.alloc(nmax / kGemmBN));
         CK(cudaMemsetAsync(m.pf_cnt.p, 0, nmax / kGemmBN * sizeof(unsigned int), g_stream));
-        ++m.pf_gen;
     }
     return 0;
 }
@@ -2839,9 +2842,8 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
     TRY(ensure_pf_scratch(m, B));
     const int pages = (total + m.page_tokens - 1) / m.page_tokens;
     if (!m.batch || m.batch->B != B || m.batch->pages_per_seq < pages) {
-        m.batch.reset(new BatchState());
+        m.batch.reset(new BatchState());   // (its B is set when all of it is there)
         BatchState& bs = *m.batch;
-        bs.B = B;
         bs.pages_per_seq = pages;
         bs.max_splits = std::max(1, std::min(m.max_splits, (2 * g_num_sms) / std::max(1, B * m.attn_heads)));
         bs.k.resize(m.layers.size());
@@ -2861,6 +2863,7 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
         TRY(bs.part_o.alloc((size_t)B * m.attn_heads * bs.max_splits * m.attn_dim));
         TRY(bs.part_ml.alloc((size_t)B * m.attn_heads * bs.max_splits * 2));
         TRY(bs.logits.alloc((size_t)B * V));
+        bs.B = B;
     }
     BatchState& bs = *m.batch;
     // The prompts' common part -- all tokens in front of the shortest prompt's last one -- goes through the layers at once, as many sequences at a
@@ -3008,7 +3011,6 @@ int ti_b200_beam_search(ti_model_t h, const int32_t* prompt, int32_t n_prompt, i
         m.beams.reset(new BeamState());
         BeamState& st = *m.beams;
         BatchState& bs = st.bs;
-        st.beam = B;
         st.pool_pages = B * pages + B;   // worst case every beam owns all its pages; + one scratch page per idle row
         bs.B = B;
         bs.pages_per_seq = pages;
@@ -3040,6 +3042,7 @@ int ti_b200_beam_search(ti_model_t h, const int32_t* prompt, int32_t n_prompt, i
         TRY(st.cand_tok.alloc((size_t)B * B));
         TRY(st.cand_cnt.alloc(B));
         TRY(st.copy_pairs.alloc((size_t)2 * B));
+        st.beam = B;   // (all of it is there)
     }
     BeamState& st = *m.beams;
     BatchState& bs = st.bs;
