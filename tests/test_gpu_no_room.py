@@ -49,6 +49,7 @@ def limits(device=NONE, pinned=NONE): shim.shim_limits(ctypes.c_size_t(device), 
 for f in ("refused", "pinned", "total", "largest"): getattr(shim, "shim_" + f).restype = ctypes.c_long
 import binusun_cases, binusun_plain
 import turboinfer_b200 as tb
+from turboinfer_b200.seq import SeqError as seq_error
 from helpers import make_model, prompt_tokens
 TOL16 = 12 * 2.0 ** -9   # a dozen roundings to bf16
 
@@ -136,4 +137,24 @@ for room in (300000, 100000, 10000, 1000):   # the failure moves forward through
         pass
 limits()
 assert np.array_equal(m.generate_batch_greedy(prompts(50), 5)[0], want)
+""")
+
+
+def test_step_after_one_without_room(shim):
+    child(shim, """
+cfg, W, m = seq([binusun_cases.attn_layer(dim=32), binusun_cases.wkv_layer(heads=2, dim=32, rank=8)], "float32")
+toks = tokens(400)
+s = m.open()
+got = [m.step([(s, toks[:60])], [range(60)])]
+for room in (300000, 100000, 20000):   # the failure moves forward through the step's buffers
+    limits(device=room)
+    try:
+        m.step([(s, toks[60:])], [range(340)])
+        raise SystemExit("no error")
+    except seq_error:
+        pass
+limits()
+got.append(m.step([(s, toks[60:70])], [range(10)]))
+got.append(m.step([(s, toks[70:])], [range(330)]))
+close(np.concatenate(got), binusun_plain.forward(cfg, W, toks), 2e-4)
 """)

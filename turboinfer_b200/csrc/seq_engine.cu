@@ -877,6 +877,7 @@ int gemm_heads(Model& m, const float* A, int lda, int a_stride, const void* W, f
 
 int ensure_scratch(Model& m, int rows, int want) {
     if (rows > m.cap_rows) {
+        m.cap_rows = 0;   // (from here on the old buffers are gone: unless all of the new ones can be had, there is no scratch)
         const size_t R = (size_t)std::max(rows, 64), D = m.d.width;
         TRY(m.x.alloc(R * D));
         if (m.n_streams > 0) TRY(m.xs.alloc(R * (size_t)m.n_streams * D));
@@ -905,6 +906,7 @@ int ensure_scratch(Model& m, int rows, int want) {
         m.cap_rows = (int)R;
     }
     if (want > m.cap_want) {
+        m.cap_want = 0;
         const size_t W = (size_t)std::max(want, 8);
         TRY(m.hn.alloc(W * m.d.width));
         TRY(m.logits.alloc(W * m.d.vocab));
