@@ -1,0 +1,38 @@
+"""Prompts of fewer than 33 tokens, whatever the size of their queries, keys and values.  A factor of a power of two on one projection and its inverse on another leaves the model as it is."""
+import numpy as np
+import pytest
+
+from helpers import make_model, prompt_tokens
+
+pytestmark = pytest.mark.gpu
+
+def scaled(meta, q, k, v):
+    w = make_model(meta, norm_jitter=0.1)
+    for l in range(meta["layers"]):
+        for name, e in (("q", q), ("k", k), ("v", v), ("o", -v)):
+            w["layers.%d.attention.%s_proj.weight" % (l, name)] *= np.float32(2.0 ** e)
+    return w
+
+
+SIZES = [(0, 0, 0), (20, -20, 0), (-20, 20, 0), (0, 0, 20), (0, 0, -14), (-12, 12, -20)]
+
+
+def load(meta, sizes, qt="Q_INT8"):
+    import turboinfer_b200 as tb
+    tb.init(0)
+    return tb.Model(meta, getattr(tb, qt), attn_mode=1, rope_mode=1, max_seq=320).load(scaled(meta, *sizes))
+
+
+@pytest.mark.parametrize("qt", ["Q_INT8", "Q_INT4"])
+@pytest.mark.parametrize("sizes", SIZES, ids=str)
+def test_short_prompts_run_token_by_token(monkeypatch, sizes, qt):
+    meta = dict(vocab=160, hidden=128, layers=2, heads=2, inter=256)
+    lens = (1, 5, 6, 7, 16, 31, 32)
+    out = []
+    for path in ("", "decode"):
+        monkeypatch.setenv("TURBOINFER_B200_PREFILL", path)
+        m = load(meta, sizes, qt)
+        out.append([m.prefill(prompt_tokens(n, meta["vocab"], offset=n)) for n in lens])
+        m.free()
+    for got, want in zip(*out):
+        assert np.array_equal(got, want)

@@ -158,3 +158,15 @@ got.append(m.step([(s, toks[60:70])], [range(10)]))
 got.append(m.step([(s, toks[70:])], [range(330)]))
 close(np.concatenate(got), binusun_plain.forward(cfg, W, toks), 2e-4)
 """)
+
+
+def test_a_short_prompt_needs_no_second_copy_of_the_weights(shim):
+    child(shim, """
+tb.init(0)
+m = llama()
+limits()
+for n in (5, 6, 8, 16, 31, 32):
+    m.prefill(prompt_tokens(n, META["vocab"]))
+    m.generate_greedy(prompt_tokens(n, META["vocab"]), 3)
+assert shim.shim_total() < 100000, shim.shim_total()   # (the weights: 2 million)
+""")

@@ -1240,26 +1240,17 @@ int pf_digits(Model& m, const float* x, const float* norm_w, int M, int K, int m
     return 0;
 }
 
-// Prompts run on the tensor-core GEMMs from a few tokens on: one pass over the layers costs about three steps of the decode engine (four
-// layers of 2048, kernel time in us: 16 tokens at once 410, one at a time 16 x 134), so that from six tokens on it is ahead with some margin.
-// The GEMMs read a byte copy of the weights, made on first use; below the 33 tokens from which the copy has always been made it must leave
-// room on the GPU.
-constexpr int kPromptGemmTokens = 6;
-bool kmajor_fits(const Model& m) {
-    size_t need = 0;
-    for (auto& ly : m.layers)
-        for (const QWeight* w : {ly.qkv.get(), ly.o.get(), ly.gateup.get(), ly.down.get()})
-            if (!w->kmajor.p) need += (size_t)(w->L.K + 512) * (w->L.N + kGemmBN);
-    if (need == 0) return true;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return false; }
-    return need + total_b / 8 <= free_b;
-}
-bool prefill_gemm_eligible(const Model& m, int M) {
-    if (M < kPromptGemmTokens || m.tp != 1 || m.cfg.attn_mode != 1 || m.cfg.rope_mode == 2 || m.attn_dim > 128 || (m.attn_dim & 3)) return false;
+// Prompts of this many tokens and more run on the tensor-core GEMMs (the reference: GEMM branch of TensorEngine::matmul from 32 rows on,
+// tensor_engine.cpp:561).  One pass over the layers would be ahead of the decode engine from about six tokens on (four layers of 2048, kernel time in us: 16
+// tokens at once 410, one at a time 16 x 134), but only once the byte copy of the weights is there: laid out inside a request of 16 tokens
+// and 64 new ones it made the first one of a model 12.8 -> 16.9 ms, on layers of 4096 13.7 -> 20.9, and it keeps an INT4 model at three times
+// its weights.  A short prompt runs token by token, whatever ran before it, so that its result does not depend on that either.
+constexpr int kPromptGemmTokens = 33;
+bool prefill_gemm_possible(const Model& m) {
+    if (m.tp != 1 || m.cfg.attn_mode != 1 || m.cfg.rope_mode == 2 || m.attn_dim > 128 || (m.attn_dim & 3)) return false;
     if (const char* e = getenv("TURBOINFER_B200_PREFILL")) if (std::string(e) == "decode") return false;
     for (auto& ly : m.layers) if (!(ly.qkv && ly.o && ly.gateup && ly.down)) return false;
-    return M >= 33 || kmajor_fits(m);
+    return true;
 }
 
 // the rows of a prefill pass: the first P tokens of n_seq sequences, one after another (tokens on the device in that order), their page tables
@@ -1544,11 +1535,11 @@ int gather_sharded_logits(Model& m, float* buf, size_t count) {
 }
 
 // ---- the prompt of a generation (forward_pass, :749): fills the KV cache; the last prompt token's logits are left in
-// m.logits (steps < n_prompt - 1 skip the lm_head).  Long prompts go through the tensor-core GEMM path (all tokens but the
-// last in one batched forward pass), short ones through the decode engine token by token.  m.prompt holds the prompt.
-int prompt_pass(Model& m, const int32_t* prompt_host, int n_prompt) {
+// m.logits (steps < n_prompt - 1 skip the lm_head).  Long prompts go through the tensor-core GEMM path in one batched forward
+// pass, short ones through the decode engine token by token.  m.prompt holds the prompt.
+int prompt_pass(Model& m, int n_prompt) {
     if (m.use_mega) {
-        if (prefill_gemm_eligible(m, n_prompt)) {
+        if (n_prompt >= kPromptGemmTokens && prefill_gemm_possible(m)) {
             TRY(prompt_gemm(m, n_prompt, 1));
         } else {
             TRY(run_mega(m, n_prompt, n_prompt, n_prompt - 1));
@@ -2406,7 +2397,7 @@ int ti_b200_prefill(ti_model_t h, const int32_t* tokens, int32_t n, float* last_
     CK(cudaMemcpyAsync(m.prompt.p, tokens, n * sizeof(int), cudaMemcpyHostToDevice, g_stream));
     StepIO io{};
     CK(cudaMemcpyAsync(m.io.p, &io, sizeof(io), cudaMemcpyHostToDevice, g_stream));
-    TRY(prompt_pass(m, tokens, n));
+    TRY(prompt_pass(m, n));
     m.host_pos = n;
     if (last_logits_host) {
         const size_t V = m.cfg.vocab;
@@ -2730,9 +2721,8 @@ int ti_b200_generate_greedy(ti_model_t h, const int32_t* prompt, int32_t n_promp
     int steps_done = 0;   // decode steps after the prompt
     if (m.use_mega) {
         // launch 1: the prompt (its last step picks token 0); launch 2: the decode loop, timed.
-        // Prompts of more than a few tokens go through the tensor-core GEMM path in one batched forward pass, the head on the last row
-        // (the reference: GEMM branch of TensorEngine::matmul from 32 rows on, tensor_engine.cpp:561).
-        if (prefill_gemm_eligible(m, n_prompt)) {
+        // Long prompts go through the tensor-core GEMM path in one batched forward pass, the head on the last row.
+        if (n_prompt >= kPromptGemmTokens && prefill_gemm_possible(m)) {
             TRY(prompt_gemm(m, n_prompt, n_new > 0 ? 1 : 0));
         } else {
             TRY(run_mega(m, n_prompt, n_prompt, n_new > 0 ? n_prompt - 1 : n_prompt));
@@ -2814,6 +2804,9 @@ static int batch_carveout() {
     return 0;
 }
 
+// rows of a batch's prompts in front of its lockstep steps from which they go through the layers at once (a step needs the byte copy of the
+// weights anyway)
+constexpr int kBatchPromptRows = 6;
 static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32_t* lens, int32_t batch, int32_t max_len, int32_t n_new,
                                int32_t* out_tokens, float* logits_last, float* decode_ms) {
     TRY(need_init());
@@ -2869,7 +2862,7 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
     // The prompts' common part -- all tokens in front of the shortest prompt's last one -- goes through the layers at once, as many sequences at a
     // time as make 4096 rows; the lockstep steps begin behind it.  (32 prompts of 6 tokens on four 7B-wide layers: five steps of 0.6 ms.)
     int done = 0;
-    if (min_len > 2 && prefill_gemm_eligible(m, B * (min_len - 1))) {
+    if (min_len > 2 && B * (min_len - 1) >= kBatchPromptRows && prefill_gemm_possible(m)) {
         const int P = min_len - 1, per = std::max(1, std::min(B, 4096 / P));
         std::vector<int> rows((size_t)B * P);
         for (int b = 0; b < B; ++b) std::copy(prompts + (size_t)b * max_len, prompts + (size_t)b * max_len + P, rows.begin() + (size_t)b * P);
@@ -3274,7 +3267,7 @@ int ti_b200_generate_sampled(ti_model_t h, const int32_t* prompt, int32_t n_prom
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    TRY(prompt_pass(m, prompt, n_prompt));
+    TRY(prompt_pass(m, n_prompt));
     CK(cudaEventRecord(e0, g_stream));
     if (m.lm_sharded && m.hist.n < (size_t)V) TRY(m.hist.alloc((size_t)V));
     int sampled = 0, passes = 0;   // tokens picked / decode passes run after the prompt
