@@ -1,10 +1,15 @@
-"""Prompts of fewer than 33 tokens, whatever the size of their queries, keys and values.  A factor of a power of two on one projection and its inverse on another leaves the model as it is."""
+"""Prompt rows whose attention is fp32 whatever the size of their queries, keys and values: the common part of a batch's prompts, and
+prompts of fewer than 33 tokens.  A factor of a power of two on one projection and its inverse on another leaves the model as it is."""
 import numpy as np
 import pytest
 
 from helpers import make_model, prompt_tokens
 
 pytestmark = pytest.mark.gpu
+
+# fp32 sums in another order: a few 2^-24 of the largest value per sum and layer
+TOL = 64 * 2.0 ** -24
+
 
 def scaled(meta, q, k, v):
     w = make_model(meta, norm_jitter=0.1)
@@ -21,6 +26,22 @@ def load(meta, sizes, qt="Q_INT8"):
     import turboinfer_b200 as tb
     tb.init(0)
     return tb.Model(meta, getattr(tb, qt), attn_mode=1, rope_mode=1, max_seq=320).load(scaled(meta, *sizes))
+
+
+@pytest.mark.parametrize("sizes", SIZES, ids=str)
+@pytest.mark.parametrize("heads,hidden", [(2, 128), (1, 128), (3, 120)])   # heads of 64, 128 and 40
+@pytest.mark.parametrize("n", [6, 33, 34, 70, 150])   # 5, 32, 33, 69 and 149 common tokens
+def test_common_part_of_a_batch(monkeypatch, sizes, heads, hidden, n):
+    meta = dict(vocab=160, hidden=hidden, layers=2, heads=heads, inter=256)
+    prompts = [prompt_tokens(n, meta["vocab"], offset=3 * b) for b in range(3)]
+    m = load(meta, sizes)
+    toks, logits, _ = m.generate_batch_greedy(np.array(prompts, dtype=np.int32), 3, want_logits=True)
+    monkeypatch.setenv("TURBOINFER_B200_PREFILL", "decode")
+    for b, p in enumerate(prompts):
+        st, sl, _ = m.generate_greedy(p, 3, want_logits=True)
+        assert np.array_equal(toks[b], st)
+        assert np.abs(logits[b] - sl[-1]).max() <= TOL * np.abs(sl[-1]).max()
+    m.free()
 
 
 @pytest.mark.parametrize("qt", ["Q_INT8", "Q_INT4"])

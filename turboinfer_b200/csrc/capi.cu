@@ -1254,8 +1254,13 @@ bool prefill_gemm_possible(const Model& m) {
 }
 
 // the rows of a prefill pass: the first P tokens of n_seq sequences, one after another (tokens on the device in that order), their page tables
-// pages_per_seq apart
-struct PrefillRows { const int* tokens; int n_seq, P; const int* tables; int pages_per_seq; };
+// pages_per_seq apart; attn32: their attention in fp32 whatever the head size (the rows of a batch's prompts, which the lockstep steps would have
+// attended in fp32: 16-bit halves hold 22 bits of a value, fewer below 2^-3, and nothing above 65504)
+struct PrefillRows { const int* tokens; int n_seq, P; const int* tables; int pages_per_seq; bool attn32; };
+// ... by a block a (row, head), the arithmetic of the lockstep step, up to this many rows a sequence, in tiles of 128 rows from there on.  Whole calls on
+// four layers (us, a block a row | tiles): 32 sequences, heads of 128, 5 rows 1311 | 1697, 16 rows 2200 | 2286, 32 rows 3883 | 3431; heads of 64, 5 rows
+// 876 | 1184, 16 rows 1464 | 1455, 32 rows 2369 | 1805; 4 sequences, 32 rows 1170 | 1113 and 800 | 739
+constexpr int kRowAttnTokens = 16;
 
 // causal attention of the rows on tcgen05: the heads' keys and values are split into tile images, as many heads at a time as the image
 // buffer takes (a buffer that cannot be had is asked for in halves, down to one head; *done stays false when there is no room for that either)
@@ -1292,6 +1297,21 @@ int prefill_gemm(Model& m, const PrefillRows& pr, Pool pool) {
     const int rope_dim = m.cfg.rope_mode == 1 ? H / m.cfg.heads : 0;
     embed_rows_kernel<<<M, 256, 0, g_stream>>>(m.tok_emb.p, pr.tokens, m.pf_x.p, H);
     ++g_launches;
+    auto row_attention = [&](int row, const float* k_pool, const float* v_pool) {   // the lockstep step's attention kernel, from this row on
+        AttnArgs a{};
+        a.q = m.pf_qkv.p + (size_t)row * 3 * H;
+        a.k_pool = k_pool;
+        a.v_pool = v_pool;
+        a.page_table = pr.tables;
+        a.page_tokens = m.page_tokens;
+        a.page_shift = log2_if_pow2(m.page_tokens);
+        a.H = H;
+        a.D = m.attn_dim;
+        a.heads = m.attn_heads;
+        a.scale = 1.0f / sqrtf((float)m.attn_dim);
+        a.out = m.pf_attn.p + (size_t)row * H;
+        return a;
+    };
     for (size_t l = 0; l < m.layers.size(); ++l) {
         Layer& ly = m.layers[l];
         float *k_pool, *v_pool;
@@ -1305,23 +1325,29 @@ int prefill_gemm(Model& m, const PrefillRows& pr, Pool pool) {
         const bool attn_fp32 = attn_sel == "fp32", attn_tf32 = attn_sel == "tf32";
         const float att_scale = 1.0f / sqrtf((float)m.attn_dim);
         bool done = false;   // tcgen05, split FP16 (attn_tc.cuh)
-        if (!attn_fp32 && !attn_tf32 && m.attn_dim == 128) TRY(prefill_attention<128>(m, k_pool, v_pool, pr, att_scale, &done));
-        if (!attn_fp32 && !attn_tf32 && m.attn_dim == 64) TRY(prefill_attention<64>(m, k_pool, v_pool, pr, att_scale, &done));
-        if (!done) {
-            for (int i = 0; i < pr.n_seq; ++i) {   // sequence by sequence
-                float* q = m.pf_qkv.p + (size_t)i * pr.P * 3 * H;
-                float* out = m.pf_attn.p + (size_t)i * pr.P * H;
-                const int* table = pr.tables + (size_t)i * pr.pages_per_seq;
-                const dim3 tc_grid(m.attn_heads, (pr.P + kTcQ - 1) / kTcQ);
-                if (attn_tf32 && m.attn_dim == 128)   // split TF32
-                    causal_attention_tc_kernel<128><<<tc_grid, kTcThreads, attn_tc_smem_bytes<128>(), g_stream>>>(q, pr.P, H, att_scale, 0, k_pool, v_pool, table, m.page_tokens, out);
-                else if (attn_tf32 && m.attn_dim == 64)
-                    causal_attention_tc_kernel<64><<<tc_grid, kTcThreads, attn_tc_smem_bytes<64>(), g_stream>>>(q, pr.P, H, att_scale, 0, k_pool, v_pool, table, m.page_tokens, out);
-                else
-                    causal_attention_kernel<<<dim3(m.attn_heads, (pr.P + kPfQ - 1) / kPfQ), kPfThreads, kPfSmemBytes, g_stream>>>(q, pr.P, H, m.attn_dim, att_scale, 0, k_pool, v_pool,
-                                                                                                                               table, m.page_tokens, out);
-                ++g_launches;
-            }
+        if (!pr.attn32 && !attn_fp32 && !attn_tf32 && m.attn_dim == 128) TRY(prefill_attention<128>(m, k_pool, v_pool, pr, att_scale, &done));
+        if (!pr.attn32 && !attn_fp32 && !attn_tf32 && m.attn_dim == 64) TRY(prefill_attention<64>(m, k_pool, v_pool, pr, att_scale, &done));
+        if (!done && pr.attn32 && pr.P <= kRowAttnTokens) {
+            AttnArgs a = row_attention(0, k_pool, v_pool);
+            a.max_splits = 1;
+            a.min_chunk = kRowAttnTokens;
+            a.zq = 3 * H;
+            a.zout = H;
+            a.ztable = pr.pages_per_seq;
+            a.prompt_rows = pr.P;
+            attn_partial_kernel<<<dim3(m.attn_heads, 1, M), kAttnThreads, m.attn_smem, g_stream>>>(a);
+            ++g_launches;
+        } else if (!done && attn_tf32 && !pr.attn32 && (m.attn_dim == 128 || m.attn_dim == 64)) {   // split TF32 (one sequence)
+            const dim3 tc_grid(m.attn_heads, (pr.P + kTcQ - 1) / kTcQ);
+            if (m.attn_dim == 128)
+                causal_attention_tc_kernel<128><<<tc_grid, kTcThreads, attn_tc_smem_bytes<128>(), g_stream>>>(m.pf_qkv.p, pr.P, H, att_scale, 0, k_pool, v_pool, pr.tables, m.page_tokens, m.pf_attn.p);
+            else
+                causal_attention_tc_kernel<64><<<tc_grid, kTcThreads, attn_tc_smem_bytes<64>(), g_stream>>>(m.pf_qkv.p, pr.P, H, att_scale, 0, k_pool, v_pool, pr.tables, m.page_tokens, m.pf_attn.p);
+            ++g_launches;
+        } else if (!done) {
+            causal_attention_kernel<<<dim3(m.attn_heads, (pr.P + kPfQ - 1) / kPfQ, pr.n_seq), kPfThreads, kPfSmemBytes, g_stream>>>(
+                m.pf_qkv.p, pr.P, H, m.attn_dim, att_scale, 0, k_pool, v_pool, pr.tables, pr.pages_per_seq, m.page_tokens, m.pf_attn.p);
+            ++g_launches;
         }
         TRY(ensure_kmajor(*ly.o));
         TRY(batch_digits(m, m.pf_attn.p, nullptr, nullptr, M, H, m_pad, ly.o->k_pad));
@@ -1346,7 +1372,7 @@ int prefill_gemm(Model& m, const PrefillRows& pr, Pool pool) {
 // A whole prompt (on the device in m.prompt) through the GEMMs, then the head on its last row: the state is what the decode engine leaves behind a prompt
 // whose last step samples (pick = 1) or does not (pick = 0).
 int prompt_gemm(Model& m, int n_prompt, int pick) {
-    TRY(prefill_gemm(m, PrefillRows{m.prompt.p, 1, n_prompt, m.page_table.p, 0}, [&](size_t l, float** k, float** v) { *k = m.layers[l].k_pool.p; *v = m.layers[l].v_pool.p; }));
+    TRY(prefill_gemm(m, PrefillRows{m.prompt.p, 1, n_prompt, m.page_table.p, 0, false}, [&](size_t l, float** k, float** v) { *k = m.layers[l].k_pool.p; *v = m.layers[l].v_pool.p; }));
     StepState st{};
     st.pos = n_prompt - 1;   // (step_finish_kernel counts the last token)
     CK(cudaMemcpyAsync(m.state.p, &st, sizeof(st), cudaMemcpyHostToDevice, g_stream));
@@ -2869,7 +2895,7 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
         if (bs.rows.n < rows.size()) TRY(bs.rows.alloc(rows.size()));
         CK(cudaMemcpyAsync(bs.rows.p, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, g_stream));
         for (int b = 0; b < B; b += per)
-            TRY(prefill_gemm(m, PrefillRows{bs.rows.p + (size_t)b * P, std::min(per, B - b), P, bs.tables.p + (size_t)b * bs.pages_per_seq, bs.pages_per_seq},
+            TRY(prefill_gemm(m, PrefillRows{bs.rows.p + (size_t)b * P, std::min(per, B - b), P, bs.tables.p + (size_t)b * bs.pages_per_seq, bs.pages_per_seq, true},
                              [&](size_t l, float** k, float** v) { *k = bs.k[l].p; *v = bs.v[l].p; }));
         done = P;
     }

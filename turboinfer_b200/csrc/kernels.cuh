@@ -340,6 +340,8 @@ struct AttnArgs {
     int zq, zout, ztable;
     size_t zpart_o, zpart_ml;
     int page_shift;          // log2(page_tokens) when it is a power of two (the fast item then needs no division), else -1
+    // > 0 (attn_partial_kernel): blockIdx.z = a prompt row; every sequence has so many, row i sees the first i + 1 tokens, the table goes by sequence
+    int prompt_rows;
 };
 TIB_HD int log2_if_pow2(int v) {
     if (v <= 0 || (v & (v - 1))) return -1;

@@ -589,7 +589,7 @@ __device__ __forceinline__ float mega_attention_lean(const AttnArgs& a, const At
 __device__ __forceinline__ AttnArgs attn_for_sequence(AttnArgs a, int z) {
     a.q += (size_t)z * a.zq;
     a.out += (size_t)z * a.zout;
-    a.page_table += (size_t)z * a.ztable;
+    a.page_table += (size_t)(a.prompt_rows > 0 ? z / a.prompt_rows : z) * a.ztable;
     a.part_o += z * a.zpart_o;
     a.part_ml += z * a.zpart_ml;
     return a;
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_partial_kernel(const AttnAr
     pdl_wait_prior_grid();       // (no-op unless launched with programmatic stream serialization: the lockstep step's graph)
     pdl_launch_dependents();
     const AttnArgs a = attn_for_sequence(a0, blockIdx.z);
-    const int t = *a.pos_ptr + a.t_bias;
+    const int t = a.prompt_rows > 0 ? (int)blockIdx.z % a.prompt_rows + 1 : *a.pos_ptr + a.t_bias;
     int nsplit, chunk;
     attn_split_range(t, a.max_splits, a.min_chunk, nsplit, chunk);
     const int j = blockIdx.y;

@@ -99,7 +99,7 @@ __global__ void rope_kv_kernel(float* qkv, int P, int H, int rope_dim, const flo
 }
 
 // Causal multi-head attention for M queries at positions pos0 .. pos0 + M - 1 over the paged cache (which already holds
-// their own K / V rows).  fp32 on the CUDA cores, organised as two register-tiled GEMMs per key tile (no per-pair
+// their own K / V rows), blockIdx.z = one of several sequences of M rows each, one after another, page tables pages_per_seq apart.  fp32 on the CUDA cores, organised as two register-tiled GEMMs per key tile (no per-pair
 // shuffles): a CTA owns 128 queries of one head; per tile of 64 keys
 //   S[128 x 64] = Q K^T   thread (ty, tx) computes 8 queries x 4 keys, reading Q and K TRANSPOSED from shared memory
 //                         ([d][query], [d][key]: two broadcast LDS.128 + one LDS.128 per 32 FMAs)
@@ -111,8 +111,11 @@ constexpr int kPfQ = 128, kPfKT = 64, kPfThreads = 256, kPfD = 128;
 constexpr size_t kPfSmemBytes = ((size_t)kPfD * kPfQ + (size_t)kPfD * kPfKT + (size_t)kPfKT * kPfD + (size_t)kPfKT * kPfQ) * sizeof(float);   // 160 KiB
 __global__ void __launch_bounds__(kPfThreads, 1) causal_attention_kernel(const float* qkv, int M, int H, int D, float scale, int pos0,
                                                                            const float* k_pool, const float* v_pool, const int* page_table,
-                                                                           int page_tokens, float* out) {
+                                                                           int pages_per_seq, int page_tokens, float* out) {
     extern __shared__ __align__(16) float pf_smem[];
+    qkv += (size_t)blockIdx.z * M * 3 * H;
+    out += (size_t)blockIdx.z * M * H;
+    page_table += (size_t)blockIdx.z * pages_per_seq;
     float* Qt = pf_smem;                       // [128 d][128 q]
     float* Kt = Qt + kPfD * kPfQ;              // [128 d][64 k]
     float* Vs = Kt + kPfD * kPfKT;             // [64 k][128 d]
