@@ -1,5 +1,5 @@
-"""Prompt rows whose attention is fp32 whatever the size of their queries, keys and values: the common part of a batch's prompts, and
-prompts of fewer than 33 tokens.  A factor of a power of two on one projection and its inverse on another leaves the model as it is."""
+"""Prompt rows whose attention is fp32 whatever the size of their queries, keys and values: the common part of a batch's prompts, and the last row
+of a prompt.  A factor of a power of two on one projection and its inverse on another leaves the model as it is."""
 import numpy as np
 import pytest
 
@@ -42,6 +42,21 @@ def test_common_part_of_a_batch(monkeypatch, sizes, heads, hidden, n):
         assert np.array_equal(toks[b], st)
         assert np.abs(logits[b] - sl[-1]).max() <= TOL * np.abs(sl[-1]).max()
     m.free()
+
+
+@pytest.mark.parametrize("sizes", SIZES, ids=str)
+@pytest.mark.parametrize("heads,hidden", [(2, 128), (1, 128), (3, 120)])
+@pytest.mark.parametrize("n", [33, 64, 129, 300])
+def test_last_row_of_a_prompt(monkeypatch, sizes, heads, hidden, n):
+    # one layer: the logits hang on the last row's attention alone
+    meta = dict(vocab=160, hidden=hidden, layers=1, heads=heads, inter=256)
+    out = []
+    for path in ("", "decode"):
+        monkeypatch.setenv("TURBOINFER_B200_PREFILL", path)
+        m = load(meta, sizes)
+        out.append(m.prefill(prompt_tokens(n, meta["vocab"])))
+        m.free()
+    assert np.abs(out[0] - out[1]).max() <= TOL * np.abs(out[1]).max()
 
 
 @pytest.mark.parametrize("qt", ["Q_INT8", "Q_INT4"])

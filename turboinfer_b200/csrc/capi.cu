@@ -1344,7 +1344,18 @@ int prefill_gemm(Model& m, const PrefillRows& pr, Pool pool) {
             else
                 causal_attention_tc_kernel<64><<<tc_grid, kTcThreads, attn_tc_smem_bytes<64>(), g_stream>>>(m.pf_qkv.p, pr.P, H, att_scale, 0, k_pool, v_pool, pr.tables, m.page_tokens, m.pf_attn.p);
             ++g_launches;
-        } else if (!done) {
+        } else if (done) {
+            // the prompt's last row again in fp32, as the decode engine attends a prompt's last token: on a model of few layers the logits hang on it
+            AttnArgs a = row_attention(M - 1, k_pool, v_pool);
+            a.pos_ptr = &m.state.p->pos;   // 0: a prompt begins behind a reset, the count follows behind the pass
+            a.t_bias = M;
+            a.max_splits = m.max_splits;
+            a.min_chunk = 64;
+            a.part_o = m.part_o.p;
+            a.part_ml = m.part_ml.p;
+            TRY(launch_step(attn_partial_kernel, dim3(m.attn_heads, m.max_splits), dim3(kAttnThreads), m.attn_smem, a));
+            TRY(launch_step(attn_combine_kernel, dim3(m.attn_heads), dim3(256), 0, a));
+        } else {
             causal_attention_kernel<<<dim3(m.attn_heads, (pr.P + kPfQ - 1) / kPfQ, pr.n_seq), kPfThreads, kPfSmemBytes, g_stream>>>(
                 m.pf_qkv.p, pr.P, H, m.attn_dim, att_scale, 0, k_pool, v_pool, pr.tables, pr.pages_per_seq, m.page_tokens, m.pf_attn.p);
             ++g_launches;
