@@ -170,3 +170,18 @@ for n in (5, 6, 8, 16, 31, 32):
     m.generate_greedy(prompt_tokens(n, META["vocab"]), 3)
 assert shim.shim_total() < 100000, shim.shim_total()   # (the weights: 2 million)
 """)
+
+
+@pytest.mark.parametrize("room,what", [(1000000, "two sequences' rows"), (500000, "one sequence's rows"), (480000, "a step's rows only")])
+def test_batch_prompts_without_room_for_their_rows(shim, room, what):
+    # four prompts of 59 common tokens at once want 1.9 MB for the inner rows, one of them 483 KB; a step of the batch wants 393 KB
+    child(shim, """
+tb.init(0)
+want2, want = alone(2, 5), alone(60, 5)
+m = llama()
+assert np.array_equal(m.generate_batch_greedy(prompts(2), 5)[0], want2)
+limits(device=%d)
+for _ in range(2): assert np.array_equal(m.generate_batch_greedy(prompts(60), 5)[0], want)
+assert shim.shim_refused() > 0
+assert np.array_equal(m.generate_batch_greedy(prompts(2), 5)[0], want2)
+""" % room)

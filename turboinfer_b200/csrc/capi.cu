@@ -2844,6 +2844,8 @@ static int batch_carveout() {
 // rows of a batch's prompts in front of its lockstep steps from which they go through the layers at once (a step needs the byte copy of the
 // weights anyway)
 constexpr int kBatchPromptRows = 6;
+// ... as many rows a pass at most: half a GB of scratch on layers of 4096 (32 prompts of 129 tokens on four of them, us at 1024 / 2048 / 4096 rows: 10977 / 10566 / 10537)
+constexpr int kBatchPassRows = 2048;
 static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32_t* lens, int32_t batch, int32_t max_len, int32_t n_new,
                                int32_t* out_tokens, float* logits_last, float* decode_ms) {
     TRY(need_init());
@@ -2897,18 +2899,26 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
     }
     BatchState& bs = *m.batch;
     // The prompts' common part -- all tokens in front of the shortest prompt's last one -- goes through the layers at once, as many sequences at a
-    // time as make 4096 rows; the lockstep steps begin behind it.  (32 prompts of 6 tokens on four 7B-wide layers: five steps of 0.6 ms.)
+    // time as make kBatchPassRows rows; the lockstep steps begin behind it.  (32 prompts of 6 tokens on four 7B-wide layers: five steps of 0.6 ms.)
+    // Rows there is no room for are halved, and without room for one sequence's the steps do it all, with the scratch of a step.
     int done = 0;
     if (min_len > 2 && B * (min_len - 1) >= kBatchPromptRows && prefill_gemm_possible(m)) {
-        const int P = min_len - 1, per = std::max(1, std::min(B, 4096 / P));
-        std::vector<int> rows((size_t)B * P);
-        for (int b = 0; b < B; ++b) std::copy(prompts + (size_t)b * max_len, prompts + (size_t)b * max_len + P, rows.begin() + (size_t)b * P);
-        if (bs.rows.n < rows.size()) TRY(bs.rows.alloc(rows.size()));
-        CK(cudaMemcpyAsync(bs.rows.p, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, g_stream));
-        for (int b = 0; b < B; b += per)
-            TRY(prefill_gemm(m, PrefillRows{bs.rows.p + (size_t)b * P, std::min(per, B - b), P, bs.tables.p + (size_t)b * bs.pages_per_seq, bs.pages_per_seq, true},
-                             [&](size_t l, float** k, float** v) { *k = bs.k[l].p; *v = bs.v[l].p; }));
-        done = P;
+        const int P = min_len - 1;
+        int per = std::max(1, std::min(B, kBatchPassRows / P));
+        bool room = false;
+        while (!(room = ensure_pf_scratch(m, per * P) == 0) && per > 1) per = (per + 1) / 2;
+        if (!room) {
+            TRY(ensure_pf_scratch(m, B));
+        } else {
+            std::vector<int> rows((size_t)B * P);
+            for (int b = 0; b < B; ++b) std::copy(prompts + (size_t)b * max_len, prompts + (size_t)b * max_len + P, rows.begin() + (size_t)b * P);
+            if (bs.rows.n < rows.size()) TRY(bs.rows.alloc(rows.size()));
+            CK(cudaMemcpyAsync(bs.rows.p, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, g_stream));
+            for (int b = 0; b < B; b += per)
+                TRY(prefill_gemm(m, PrefillRows{bs.rows.p + (size_t)b * P, std::min(per, B - b), P, bs.tables.p + (size_t)b * bs.pages_per_seq, bs.pages_per_seq, true},
+                                 [&](size_t l, float** k, float** v) { *k = bs.k[l].p; *v = bs.v[l].p; }));
+            done = P;
+        }
     }
     bool regraph = false;
     if (bs.out.n < (size_t)B * n_new) {
