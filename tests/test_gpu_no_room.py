@@ -185,3 +185,19 @@ for _ in range(2): assert np.array_equal(m.generate_batch_greedy(prompts(60), 5)
 assert shim.shim_refused() > 0
 assert np.array_equal(m.generate_batch_greedy(prompts(2), 5)[0], want2)
 """ % room)
+
+
+def test_split_keys_of_visible_pages_only(shim):
+    # portions of 128 rows with windows of 100 and 300 behind up to 9000 tokens: the pages in front of the windows are neither split nor stored
+    child(shim, """
+layers = [binusun_cases.attn_layer(heads=4, kv_heads=4, dim=64, vdim=64, rot_dims=8, window=w) for w in (100, 300)]
+cfg, W, m = seq(layers, "bfloat16", max_tokens=2 * 9088, max_seqs=2)
+toks = tokens(9000)
+s = m.open()
+m.step([(s, toks[:512])])
+limits()
+for i in range(512, 8704, 512): m.step([(s, toks[i:i + 512])])
+got = m.step([(s, toks[8704:8832])], [range(128)])
+assert shim.shim_largest() < 3000000, shim.shim_largest()   # 512 + 300 rows in 14 pages of four heads of 32 KB; all pages: 18 MB
+close(got, binusun_plain.forward(cfg, W, toks[8000:8832])[-128:], TOL16)   # (the windows reach 398 tokens back)
+""")

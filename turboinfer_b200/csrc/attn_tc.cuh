@@ -54,7 +54,7 @@ template <int DK, int DV, typename Src>
 __global__ void __launch_bounds__(256) kv_images_kernel(const Src src, uint8_t* images) {
     const int g = src.g0 + blockIdx.y;
     typename Src::Tile tile;
-    if (!src.tile(blockIdx.x, tile)) return;   // (no row of the step sees a key of this tile)
+    src.tile(blockIdx.x, tile);
     uint8_t* rec = images + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * at_record_bytes(DK, DV);
     // a thread takes eight coordinates of a key: two 16-byte loads, one 16-byte store into each half
     for (int i = threadIdx.x; i < kAtKT * (DK + DV) / 8; i += 256) {

@@ -437,10 +437,9 @@ struct PrefillKeys {   // kv_images_kernel: key t of a prompt; the prompts (P to
     const int* page_table;
     int pages_per_seq, page_tokens, H, d, dv, P, kt, g0;
     struct Tile { const int* table; int t0; };
-    __device__ bool tile(int x, Tile& t) const {
+    __device__ void tile(int x, Tile& t) const {
         t.table = page_table + (size_t)(x / kt) * pages_per_seq;
         t.t0 = x % kt * kAtKT;
-        return true;
     }
     __device__ const float* row(const Tile& tile, int r, int g, bool is_v) const {
         const int t = tile.t0 + r;

@@ -13,21 +13,19 @@ namespace seq {
 
 constexpr int kAttnTcTile = kAtQ;   // 128 rows a block
 
-struct SeqKeys {   // kv_images_kernel: the pages (64 tokens) of the step's portions, one after another
+struct SeqKeys {   // kv_images_kernel: the pages (64 tokens) that the step's portions see, one after another
     StepMeta m;
     AttnShape s;
     const int* pages;   // [2 x] = entry, [2 x + 1] = page of its sequence
     const float *k_pool, *v_pool;
     int d, dv, g0;
     struct Tile { size_t tok0; int t0, lo, last; };
-    __device__ bool tile(int x, Tile& t) const {
+    __device__ void tile(int x, Tile& t) const {
         const int e = pages[2 * x], p = pages[2 * x + 1], pos0 = m.ent_pos0[e];
         t.t0 = p * kPageTokens;
         t.lo = attn_first_key(s, pos0);
         t.last = pos0 + m.ent_row0[e + 1] - m.ent_row0[e] - 1;
-        if (t.t0 + kPageTokens - 1 < t.lo) return false;
         t.tok0 = (size_t)m.page_table[(size_t)m.ent_slot[e] * m.table_stride + p] * kPageTokens;
-        return true;
     }
     __device__ const float* row(const Tile& t, int r, int g, bool is_v) const {
         if (t.t0 + r < t.lo || t.t0 + r > t.last) return nullptr;
@@ -38,7 +36,7 @@ struct SeqAttn {
     StepMeta m;
     AttnShape s;
     const int* tiles;
-    const int* image0;   // [entries]: the record of an entry's page 0
+    const int* image0;   // [entries]: where the record of an entry's page 0 would lie (negative when its first pages have none)
     const float* qkvg;
     float* out;
     int d, dv, group, h0;

@@ -274,6 +274,7 @@ struct Model {
     DevBuf<int> meta, picks;
     DevBuf<float> wkv_M;         // chunked recurrence: products inside the chunks of 16 tokens, then the chunks' decays
     DevBuf<uint8_t> kv_images;   // split keys and values of the portions' attention (one layer run's, rewritten by the next)
+    std::vector<std::pair<int, int>> spans;   // the different (window, chunk) of the attention layers
     DevBuf<__nv_bfloat16> abf;   // bf16 copy of a product's activations for the tcgen05 path: [rows][max_k]
     DevBuf<int> attn_arrived;    // split-key attention: finished splits of a (row, head), zero between launches
     DevBuf<float> attn_part;     // split-key attention partials: [rows][heads][splits][vdim + 2]
@@ -1059,17 +1060,28 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
             r0 += counts[e];
         }
     }
-    // the split key tiles of the portions' attention: every page of a portion's sequence, entry by entry
+    // the split key tiles of the portions' attention, a list for every span: of each portion's sequence the pages from the first one that the portion's
+    // first row sees, entry by entry; image0: where an entry's page 0 would lie
+    struct KeyTiles { int first = 0, n = 0; const int *pages = nullptr, *image0 = nullptr; };
+    std::vector<KeyTiles> spans;
     std::vector<int> ktiles, image0;
     if (!tiles128.empty() && m.d.mode == TI_SEQ_BF16) {
-        image0.assign(E, 0);
-        for (int e = 0; e < E; ++e) {
-            if (counts[e] < kAttnTiledMinRows) continue;
-            image0[e] = (int)ktiles.size() / 2;
-            for (int p = 0; p < (m.seqs[seqs[e]].len + counts[e] + kPageTokens - 1) / kPageTokens; ++p) { ktiles.push_back(e); ktiles.push_back(p); }
+        for (auto& [window, chunk] : m.spans) {
+            KeyTiles k;
+            k.first = (int)ktiles.size() / 2;
+            AttnShape s{};
+            s.window = window;
+            s.chunk = chunk;
+            for (int e = 0; e < E; ++e) {
+                const int pos0 = m.seqs[seqs[e]].len, page0 = attn_first_key(s, pos0) / kPageTokens;
+                image0.push_back((int)ktiles.size() / 2 - k.first - page0);
+                if (counts[e] < kAttnTiledMinRows) continue;
+                for (int p = page0; p < (pos0 + counts[e] + kPageTokens - 1) / kPageTokens; ++p) { ktiles.push_back(e); ktiles.push_back(p); }
+            }
+            k.n = (int)ktiles.size() / 2 - k.first;
+            spans.push_back(k);
         }
     }
-    const int n_ktiles = (int)ktiles.size() / 2;
     const size_t n_xtable = xpages.empty() ? 0 : (size_t)m.seqs.size() * stride;
     const size_t n_meta = (size_t)3 * T + (size_t)(E + 1) + 2 * (size_t)E + (size_t)std::max(n_out, 1) + (size_t)m.seqs.size() * stride +
                           (size_t)3 * T + 4 + mtiles.size() + row_tile.size() + xpages.size() + n_xtable + ktiles.size() + image0.size();
@@ -1145,6 +1157,10 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     const int* d_xtable = d_xpages + xpages.size();
     const int* d_ktiles = d_xtable + n_xtable;
     const int* d_image0 = d_ktiles + ktiles.size();
+    for (size_t i = 0; i < spans.size(); ++i) {
+        spans[i].pages = d_ktiles + 2 * (size_t)spans[i].first;
+        spans[i].image0 = d_image0 + i * E;
+    }
     sm.table_stride = stride;
     sm.T = T;
     sm.E = E;
@@ -1255,8 +1271,13 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     auto h3_size = [](const AttnShape& s) { return s.dim <= 128 && s.vdim <= 128 && s.dim % 4 == 0 && s.vdim % 4 == 0 && s.v_ld == 0; };
     // keys and values are split into tile images first: as many heads at a time as the image buffer takes (a buffer that cannot be had is
     // asked for in halves, down to one head; 0: no room for one either)
+    auto key_tiles = [&](const AttnShape& s) -> const KeyTiles& {
+        size_t i = 0;
+        while (m.spans[i] != std::make_pair(s.window, s.chunk)) ++i;   // (every attention layer's is among them)
+        return spans[i];
+    };
     auto h3_heads = [&](const AttnShape& s) {
-        const int dk = at_pad(s.dim), dv = at_pad(s.vdim);
+        const int dk = at_pad(s.dim), dv = at_pad(s.vdim), n_ktiles = key_tiles(s).n;
         int per = at_heads_per_launch(s.kv_heads, n_ktiles, dk, dv, kAtImageBudget);
         while (m.kv_images.n < (size_t)per * n_ktiles * at_record_bytes(dk, dv)) {
             if (m.kv_images.alloc((size_t)per * n_ktiles * at_record_bytes(dk, dv)) == 0) break;
@@ -1267,14 +1288,15 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     };
     auto h3_attention = [&](const StepMeta& sm, const AttnShape& s, const float* q, const float* kp, const float* vp, float* out) -> int {   // the portions' tiles
         const int dk = at_pad(s.dim), dv = at_pad(s.vdim), group = s.heads / s.kv_heads, per = h3_heads(s);
+        const KeyTiles& kt = key_tiles(s);
         if (per == 0) return 1;
         for (int g0 = 0; g0 < s.kv_heads; g0 += per) {
             const int ng = std::min(per, s.kv_heads - g0);
-            const SeqKeys keys{sm, s, d_ktiles, kp, vp, s.dim, s.vdim, g0};
-            const SeqAttn shape{sm, s, d_tiles128, d_image0, q, out, s.dim, s.vdim, group, g0 * group};
+            const SeqKeys keys{sm, s, kt.pages, kp, vp, s.dim, s.vdim, g0};
+            const SeqAttn shape{sm, s, d_tiles128, kt.image0, q, out, s.dim, s.vdim, group, g0 * group};
 #define TI_AT_CASE(K, V)                                                                                                                               \
     {                                                                                                                                                  \
-        kv_images_kernel<K, V, SeqKeys><<<dim3(n_ktiles, ng), 256, 0, g_stream>>>(keys, m.kv_images.p);                                                \
+        kv_images_kernel<K, V, SeqKeys><<<dim3(kt.n, ng), 256, 0, g_stream>>>(keys, m.kv_images.p);                                                \
         attn_tc_kernel<K, V, SeqAttn><<<dim3(ng * group, n_tiles128), kAtThreads, attn_tc_smem_bytes5<K, V>(), g_stream>>>(shape, m.kv_images.p, m.err.p); \
     }
             if (dk == 64 && dv == 64) TI_AT_CASE(64, 64)
@@ -2669,6 +2691,10 @@ int ti_seq_model_finalize(ti_seq_model_t h) {
         }
     }
     m.max_k = std::max({m.max_k, 2 * D, m.max_att, m.max_ff, m.max_rank, D});
+    for (const LayerW& L : m.layers) {
+        const std::pair<int, int> span(L.d.window, L.d.chunk);
+        if ((L.d.mixer == TI_SEQ_MIXER_ATTENTION || L.d.mixer == TI_SEQ_MIXER_LATENT) && std::find(m.spans.begin(), m.spans.end(), span) == m.spans.end()) m.spans.push_back(span);
+    }
     TRY(m.err.alloc(1));
     CK(cudaMemset(m.err.p, 0, sizeof(int)));
     if (m.stage.open() != cudaSuccess) cudaGetLastError();   // (logits then take the driver's own way)

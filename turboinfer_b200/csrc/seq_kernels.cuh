@@ -869,9 +869,9 @@ struct AttnShape {
     int chunk = 0;                    // > 0: a row sees no key in front of its own chunk of positions (pos / chunk * chunk)
 };
 // the first key position a row at `pos` sees (never later for an earlier row)
-__device__ __forceinline__ int attn_first_key(const AttnShape& s, int pos) {
-    int lo = s.window > 0 ? max(pos - s.window + 1, 0) : 0;
-    if (s.chunk > 0) lo = max(lo, pos / s.chunk * s.chunk);
+__host__ __device__ __forceinline__ int attn_first_key(const AttnShape& s, int pos) {
+    int lo = s.window > 0 && pos - s.window + 1 > 0 ? pos - s.window + 1 : 0;
+    if (s.chunk > 0 && pos / s.chunk * s.chunk > lo) lo = pos / s.chunk * s.chunk;
     return lo;
 }
 __device__ __forceinline__ size_t attn_out_stride(const AttnShape& s) { return s.out_ld ? (size_t)s.out_ld : (size_t)s.heads * s.vdim; }
