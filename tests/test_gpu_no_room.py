@@ -201,3 +201,38 @@ got = m.step([(s, toks[8704:8832])], [range(128)])
 assert shim.shim_largest() < 3000000, shim.shim_largest()   # 512 + 300 rows in 14 pages of four heads of 32 KB; all pages: 18 MB
 close(got, binusun_plain.forward(cfg, W, toks[8000:8832])[-128:], TOL16)   # (the windows reach 398 tokens back)
 """)
+
+
+@pytest.mark.parametrize("room", [140000, 100000])   # two key/value heads of four pages: 262 KB; one: 131 KB, then none
+def test_attention_without_room_for_split_keys(shim, room):
+    child(shim, """
+cfg, W, m = seq([binusun_cases.attn_layer(heads=4, kv_heads=2, dim=64, vdim=64, rot_dims=8, window=1000) for _ in range(3)], "bfloat16")
+toks = tokens(256)
+s = m.open()
+got = [m.step([(s, toks[:128])], [range(128)])]
+limits(device=%d)
+got.append(m.step([(s, toks[128:])], [range(128)]))
+assert 0 < shim.shim_refused() <= 2, shim.shim_refused()   # (asked once a step, not once a layer)
+close(np.concatenate(got), binusun_plain.forward(cfg, W, toks), TOL16)
+""" % room)
+
+
+def test_prompt_without_room_for_split_keys(shim):
+    # a batch leaves scratch of 236 rows behind (and no images): the prompt then only lacks room for its keys and values, 262 KB for all four heads
+    child(shim, """
+tb.init(0)
+os.environ["TURBOINFER_B200_PREFILL"] = "decode"
+m = llama()
+want = m.prefill(prompt_tokens(128, META["vocab"]))
+m.free()
+del os.environ["TURBOINFER_B200_PREFILL"]
+for room in (140000, 70000, 60000):   # two heads, one, none
+    m = llama()
+    m.generate_batch_greedy(prompts(60), 2)
+    limits(device=room)
+    got = m.prefill(prompt_tokens(128, META["vocab"]))
+    assert shim.shim_refused() in (1, 2, 3), shim.shim_refused()   # (asked once a prompt, not once a layer)
+    limits()
+    close(got, want, 64 * 2.0 ** -24)
+    m.free()
+""")

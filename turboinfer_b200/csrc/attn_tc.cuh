@@ -397,5 +397,23 @@ inline int at_heads_per_launch(int kv_heads, size_t key_tiles, int dk, int dv, s
     return (int)std::max<size_t>(1, std::min<size_t>(kv_heads, budget / one));
 }
 constexpr size_t kAtImageBudget = (size_t)256 << 20;
+// ... and the buffer that holds them, a power of two of bytes while that is within the budget: contexts that grow by a page a step must not ask for a new one
+// each time.  One that cannot be had is asked for in halves, down to one head (0: no room for that either).  `refused`: the smallest size that
+// was not to be had in this pass over the layers, which is not asked for again
+template <typename Buf>
+int at_heads_with_room(Buf& images, int kv_heads, size_t key_tiles, int dk, int dv, size_t& refused) {
+    const size_t one = key_tiles * at_record_bytes(dk, dv);
+    for (int per = at_heads_per_launch(kv_heads, key_tiles, dk, dv, kAtImageBudget);; per = (per + 1) / 2) {
+        if (images.n >= per * one) return per;
+        size_t whole = 1;
+        while (whole < per * one) whole *= 2;
+        for (size_t size : {whole, per * one}) {
+            if (size >= refused || (size == whole && whole > kAtImageBudget)) continue;
+            if (images.alloc(size) == 0) return per;
+            refused = size;
+        }
+        if (per == 1) return 0;
+    }
+}
 
 }  // namespace tib

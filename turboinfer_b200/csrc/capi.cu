@@ -1263,16 +1263,12 @@ struct PrefillRows { const int* tokens; int n_seq, P; const int* tables; int pag
 constexpr int kRowAttnTokens = 16;
 
 // causal attention of the rows on tcgen05: the heads' keys and values are split into tile images, as many heads at a time as the image
-// buffer takes (a buffer that cannot be had is asked for in halves, down to one head; *done stays false when there is no room for that either)
+// buffer takes (*done stays false when there is no room for one)
 template <int DH>
-int prefill_attention(Model& m, const float* k_pool, const float* v_pool, const PrefillRows& pr, float scale, bool* done) {
+int prefill_attention(Model& m, const float* k_pool, const float* v_pool, const PrefillRows& pr, float scale, size_t& refused, bool* done) {
     const int H = m.cfg.hidden, heads = m.attn_heads, kt = (pr.P + kAtKT - 1) / kAtKT, tiles = pr.n_seq * kt;
-    int per = at_heads_per_launch(heads, tiles, DH, DH, kAtImageBudget);
-    while (m.pf_images.n < (size_t)per * tiles * at_record_bytes(DH, DH)) {
-        if (m.pf_images.alloc((size_t)per * tiles * at_record_bytes(DH, DH)) == 0) break;
-        if (per == 1) return 0;
-        per = (per + 1) / 2;
-    }
+    const int per = at_heads_with_room(m.pf_images, heads, tiles, DH, DH, refused);
+    if (per == 0) return 0;
     *done = true;
     for (int h0 = 0; h0 < heads; h0 += per) {
         const int nh = std::min(per, heads - h0);
@@ -1312,6 +1308,7 @@ int prefill_gemm(Model& m, const PrefillRows& pr, Pool pool) {
         a.out = m.pf_attn.p + (size_t)row * H;
         return a;
     };
+    size_t refused = SIZE_MAX;   // (no such size of the image buffer was refused yet)
     for (size_t l = 0; l < m.layers.size(); ++l) {
         Layer& ly = m.layers[l];
         float *k_pool, *v_pool;
@@ -1325,8 +1322,8 @@ int prefill_gemm(Model& m, const PrefillRows& pr, Pool pool) {
         const bool attn_fp32 = attn_sel == "fp32", attn_tf32 = attn_sel == "tf32";
         const float att_scale = 1.0f / sqrtf((float)m.attn_dim);
         bool done = false;   // tcgen05, split FP16 (attn_tc.cuh)
-        if (!pr.attn32 && !attn_fp32 && !attn_tf32 && m.attn_dim == 128) TRY(prefill_attention<128>(m, k_pool, v_pool, pr, att_scale, &done));
-        if (!pr.attn32 && !attn_fp32 && !attn_tf32 && m.attn_dim == 64) TRY(prefill_attention<64>(m, k_pool, v_pool, pr, att_scale, &done));
+        if (!pr.attn32 && !attn_fp32 && !attn_tf32 && m.attn_dim == 128) TRY(prefill_attention<128>(m, k_pool, v_pool, pr, att_scale, refused, &done));
+        if (!pr.attn32 && !attn_fp32 && !attn_tf32 && m.attn_dim == 64) TRY(prefill_attention<64>(m, k_pool, v_pool, pr, att_scale, refused, &done));
         if (!done && pr.attn32 && pr.P <= kRowAttnTokens) {
             AttnArgs a = row_attention(0, k_pool, v_pool);
             a.max_splits = 1;

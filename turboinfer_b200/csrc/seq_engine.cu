@@ -1269,22 +1269,15 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     if (front) TRY(hyper(0, -1));
     // paged softmax attention of all rows of the step (prompt portions in tiles, the other rows one by one or split over their keys)
     auto h3_size = [](const AttnShape& s) { return s.dim <= 128 && s.vdim <= 128 && s.dim % 4 == 0 && s.vdim % 4 == 0 && s.v_ld == 0; };
-    // keys and values are split into tile images first: as many heads at a time as the image buffer takes (a buffer that cannot be had is
-    // asked for in halves, down to one head; 0: no room for one either)
+    // keys and values are split into tile images first: as many heads at a time as the image buffer takes (0: no room for one)
+    size_t refused = SIZE_MAX;
     auto key_tiles = [&](const AttnShape& s) -> const KeyTiles& {
         size_t i = 0;
         while (m.spans[i] != std::make_pair(s.window, s.chunk)) ++i;   // (every attention layer's is among them)
         return spans[i];
     };
     auto h3_heads = [&](const AttnShape& s) {
-        const int dk = at_pad(s.dim), dv = at_pad(s.vdim), n_ktiles = key_tiles(s).n;
-        int per = at_heads_per_launch(s.kv_heads, n_ktiles, dk, dv, kAtImageBudget);
-        while (m.kv_images.n < (size_t)per * n_ktiles * at_record_bytes(dk, dv)) {
-            if (m.kv_images.alloc((size_t)per * n_ktiles * at_record_bytes(dk, dv)) == 0) break;
-            if (per == 1) return 0;
-            per = (per + 1) / 2;
-        }
-        return per;
+        return at_heads_with_room(m.kv_images, s.kv_heads, key_tiles(s).n, at_pad(s.dim), at_pad(s.vdim), refused);
     };
     auto h3_attention = [&](const StepMeta& sm, const AttnShape& s, const float* q, const float* kp, const float* vp, float* out) -> int {   // the portions' tiles
         const int dk = at_pad(s.dim), dv = at_pad(s.vdim), group = s.heads / s.kv_heads, per = h3_heads(s);
