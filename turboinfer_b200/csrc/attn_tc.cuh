@@ -288,15 +288,14 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
                 bar_sync(2 + q, 64);
                 const float mn = fmaxf(m, fmaxf(mine, pmax[(half ^ 1) * kAtQ + r]));
                 bar_sync(2 + q, 64);   // (both have read: the place is free for the next tile)
-                constexpr float kLog2e = 1.4426950408889634f;
-                const float base = mn == -INFINITY ? 0.f : mn * kLog2e;   // (nothing visible so far: exp(-inf) = 0 everywhere)
+                const float base = mn == -INFINITY ? 0.f : mn;   // (nothing visible so far: exp(-inf) = 0 everywhere)
                 float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int j = 0; j < kAtHalf; ++j) {
-                    sc[j] = exp2f(fmaf(sc[j], kLog2e, -base));
+                    sc[j] = expf(sc[j] - base);   // (in base 2 with a rounded maximum, neighbouring tiles of large scores would not agree on it)
                     sum[j & 3] += sc[j];
                 }
-                f = mn == -INFINITY ? 1.f : exp2f((m - mn) * kLog2e);
+                f = mn == -INFINITY ? 1.f : expf(m - mn);
                 l = l * f + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
                 m = mn;
             }
