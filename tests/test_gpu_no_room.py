@@ -236,3 +236,32 @@ for room in (140000, 70000, 60000):   # two heads, one, none
     close(got, want, 64 * 2.0 ** -24)
     m.free()
 """)
+
+
+def test_results_without_a_pinned_buffer(shim):
+    child(shim, """
+limits(pinned=300000)
+tb.init(0)
+m = llama()
+got = m.prefill(prompt_tokens(20, META["vocab"]))
+cfg, W, e = seq([binusun_cases.attn_layer(dim=32)], "float32")
+toks = tokens(40)
+out = e.step([(e.open(), toks)], [range(40)])
+assert shim.shim_refused() >= 2, shim.shim_refused()   # (one buffer a library)
+close(out, binusun_plain.forward(cfg, W, toks), 2e-4)
+tb.shutdown()
+limits()
+tb.init(0)
+assert np.array_equal(got, llama().prefill(prompt_tokens(20, META["vocab"])))
+""")
+
+
+def test_models_pin_no_memory_of_their_own(shim):
+    child(shim, """
+tb.init(0)
+first = llama()
+_, _, e = seq([binusun_cases.attn_layer(dim=32)], "float32")
+limits()
+keep = [llama() for _ in range(3)] + [seq([binusun_cases.attn_layer(dim=32)], "float32")[2] for _ in range(3)]
+assert shim.shim_pinned() == 0, shim.shim_pinned()
+""")

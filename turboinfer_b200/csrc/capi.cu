@@ -36,6 +36,7 @@ uint64_t g_launches = 0;
 bool g_use_pdl = false;
 static int kEosChunk = 32;   // decode steps per launch when the generation may end early (stop_on_eos); TURBOINFER_B200_EOS_CHUNK for experiments
 bool g_attr_done = false;
+StageOut g_stage;           // logits on their way to the caller
 bool g_batch_carveout_done = false;   // the batched step's uniform carve-out preference (reset by shutdown, like g_attr_done)
 
 // ---- tensor parallelism: NCCL is loaded at run time (dlopen), so the library has no link-time dependency on it ----
@@ -397,7 +398,6 @@ struct Model {
     int pf_cap = 0;
     float last_prefill_ms = 0.f;   // CUDA-event time of the prompt phase of the last generate call
     DevBuf<float> pf_x, pf_qkv, pf_attn, pf_gu, pf_act, pf_sx;
-    StageOut stage;              // logits on their way to the caller
     DevBuf<uint8_t> pf_images;   // split keys and values of the prefill attention
     DevBuf<int8_t> pf_planes;
     DevBuf<long long> pf_sxf;
@@ -1791,6 +1791,7 @@ int ti_b200_init(int device) {
         *g_gemm_err = 0;
         CK(cudaHostGetDevicePointer(&g_gemm_err_dev, g_gemm_err, 0));
     }
+    if (g_stage.open() != cudaSuccess) cudaGetLastError();   // (logits then take the driver's own way)
     g_device = device;
     const char* pdl = getenv("TURBOINFER_B200_PDL");
     g_use_pdl = pdl ? atoi(pdl) != 0 : true;   // programmatic dependent launch of the stand-alone GEMV: on unless TURBOINFER_B200_PDL=0
@@ -1812,6 +1813,7 @@ int ti_b200_shutdown(void) {
         g_tp_size = 1;
         g_tp_rank = 0;
     }
+    g_stage.close();
     cudaStreamDestroy(g_stream);
     g_stream = nullptr;
     g_device = -1;
@@ -2439,9 +2441,9 @@ int ti_b200_prefill(ti_model_t h, const int32_t* tokens, int32_t n, float* last_
             if (m.hist.n < V) TRY(m.hist.alloc(V));
             CK(cudaMemcpyAsync(m.hist.p, m.logits.p, V * 4, cudaMemcpyDeviceToDevice, g_stream));
             TRY(gather_sharded_logits(m, m.hist.p, V));
-            CK(m.stage.copy(last_logits_host, m.hist.p, V * 4, g_stream));
+            CK(g_stage.copy(last_logits_host, m.hist.p, V * 4, g_stream));
         } else {
-            CK(m.stage.copy(last_logits_host, m.logits.p, V * 4, g_stream));
+            CK(g_stage.copy(last_logits_host, m.logits.p, V * 4, g_stream));
         }
     }
     TRY(sync_stream());
@@ -2615,7 +2617,6 @@ int ti_b200_model_finalize(ti_model_t h) {
         TRY(capture_graph(m, true, &m.graph_decode));
         TRY(capture_graph(m, false, &m.graph_prefill));
     }
-    if (m.stage.open() != cudaSuccess) cudaGetLastError();   // (logits then take the driver's own way)
     m.finalized = true;
     m.host_pos = 0;
     return 0;
@@ -2709,9 +2710,9 @@ int ti_b200_decode_step(ti_model_t h, int32_t token, float* logits_host, int32_t
             if (m->hist.n < (size_t)m->cfg.vocab) TRY(m->hist.alloc((size_t)m->cfg.vocab));
             CK(cudaMemcpyAsync(m->hist.p, m->logits.p, (size_t)m->cfg.vocab * 4, cudaMemcpyDeviceToDevice, g_stream));
             TRY(gather_sharded_logits(*m, m->hist.p, (size_t)m->cfg.vocab));
-            CK(m->stage.copy(logits_host, m->hist.p, (size_t)m->cfg.vocab * 4, g_stream));
+            CK(g_stage.copy(logits_host, m->hist.p, (size_t)m->cfg.vocab * 4, g_stream));
         } else {
-            CK(m->stage.copy(logits_host, m->logits.p, (size_t)m->cfg.vocab * 4, g_stream));
+            CK(g_stage.copy(logits_host, m->logits.p, (size_t)m->cfg.vocab * 4, g_stream));
         }
     }
     int tok = 0;
@@ -2801,7 +2802,7 @@ int ti_b200_generate_greedy(ti_model_t h, const int32_t* prompt, int32_t n_promp
     if (have > 0) CK(cudaMemcpyAsync(toks.data(), m.out_tokens.p, have * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
     if (logits_host && have > 0) {
         TRY(gather_sharded_logits(m, m.hist.p, (size_t)have * V));
-        CK(m.stage.copy(logits_host, m.hist.p, (size_t)have * V * 4, g_stream));
+        CK(g_stage.copy(logits_host, m.hist.p, (size_t)have * V * 4, g_stream));
     }
     TRY(sync_stream());
     float ms = 0.f;
@@ -2963,7 +2964,7 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
     for (int i = 1; i < n_new; ++i) TRY(run(true));
     CK(cudaEventRecord(e1, g_stream));
     CK(cudaMemcpyAsync(out_tokens, bs.out.p, (size_t)B * n_new * sizeof(int), cudaMemcpyDeviceToHost, g_stream));
-    if (logits_last) CK(m.stage.copy(logits_last, bs.logits.p, (size_t)B * V * sizeof(float), g_stream));
+    if (logits_last) CK(g_stage.copy(logits_last, bs.logits.p, (size_t)B * V * sizeof(float), g_stream));
     TRY(sync_stream());
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));

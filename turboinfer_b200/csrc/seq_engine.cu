@@ -39,6 +39,7 @@ thread_local std::string g_err;
 int g_device = -1, g_num_sms = 0;
 cudaStream_t g_stream = nullptr;
 uint64_t g_launches = 0;
+StageOut g_stage;               // logits on their way to the caller
 size_t g_smem_optin = 0;
 bool g_use_tiled_attn = true;   // TURBOINFER_B200_SEQ_TILED_ATTN=0: every row goes through the row-at-a-time attention kernel
 constexpr int kAttnTiledMinRows = 8;   // portions at least this long are cut into attention tiles
@@ -288,7 +289,6 @@ struct Model {
     int max_heads_v = 0;         // max over attention layers of heads * (vdim + 2)
     DevBuf<int> err;             // device flag: a bounded wait in a kernel ran out
     int max_k = 0;
-    StageOut stage;
     int* meta_host = nullptr;
     size_t meta_host_cap = 0;
     int max_proj = 0, max_att = 0, max_ff = 0, max_rank = 0;
@@ -1987,7 +1987,7 @@ int run_step(Model& m, int E, const int32_t* seqs, const int32_t* counts, const 
     // (the flag goes to pinned memory behind the step's table: the copies in front of the logits must not wait for the stream)
     int* kerr_host = m.meta_host + m.meta_host_cap;
     CK(cudaMemcpyAsync(kerr_host, m.err.p, sizeof(int), cudaMemcpyDeviceToHost, g_stream));
-    if (!smp.on && n_want > 0 && logits_host) CK(m.stage.copy(logits_host, m.logits.p, (size_t)n_want * V * sizeof(float), g_stream));
+    if (!smp.on && n_want > 0 && logits_host) CK(g_stage.copy(logits_host, m.logits.p, (size_t)n_want * V * sizeof(float), g_stream));
     CK(cudaStreamSynchronize(g_stream));
     const int kerr = *kerr_host;
     if (kerr) return fail("step: a bounded wait inside a kernel ran out (tensor-core product pipeline)");
@@ -2139,6 +2139,7 @@ int ti_seq_init(int device) {
     g_num_sms = p.multiProcessorCount;
     g_smem_optin = std::min<size_t>(p.sharedMemPerBlockOptin, 200 * 1024);
     if (!g_stream) CK(cudaStreamCreateWithFlags(&g_stream, cudaStreamNonBlocking));
+    if (g_stage.open() != cudaSuccess) cudaGetLastError();   // (logits then take the driver's own way)
     CK(cudaFuncSetAttribute(gemv_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_smem_optin));
     CK(cudaFuncSetAttribute(gemv_rows_mma_kernel<COLS_PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_smem_optin));
     CK(cudaFuncSetAttribute(gemv_rows_mma_kernel<COLS_SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_smem_optin));
@@ -2690,7 +2691,6 @@ int ti_seq_model_finalize(ti_seq_model_t h) {
     }
     TRY(m.err.alloc(1));
     CK(cudaMemset(m.err.p, 0, sizeof(int)));
-    if (m.stage.open() != cudaSuccess) cudaGetLastError();   // (logits then take the driver's own way)
     CK(cudaEventCreate(&m.ev0));
     CK(cudaEventCreate(&m.ev1));
     m.finalized = true;
