@@ -22,6 +22,7 @@
 #include "prefill.cuh"
 #include "batch.cuh"
 #include "stage_out.cuh"
+#include "err_words.h"
 #include "sampling.cuh"
 
 using namespace tib;
@@ -73,7 +74,12 @@ int fail(const char* fmt, ...) {
         if (rc_ != 0) return rc_; \
     } while (0)
 
+ErrWords g_err_words;
+thread_local int g_call_word = 0;   // the error word of the model that this thread's call is about: need_init() takes it back, get_model() sets it
+int* call_err() { return g_err_words.dev + g_call_word; }
+
 int need_init() {
+    g_call_word = 0;
     if (g_device < 0) return fail("ti_b200: not initialised -- call ti_b200_init(device) first (no CPU fallback exists)");
     return 0;
 }
@@ -145,16 +151,11 @@ int pick_stages(const QLayout& L, int* stages, size_t* smem) {
     return fail("GEMV K=%d does not fit shared memory (x digits need %d KiB)", L.K, layout_kpad(L) * 3 / 1024);
 }
 
-// A tensor-core GEMM whose bounded waits ran out leaves a 1 in this mapped host word (its results are then not to be used); read behind
+// A tensor-core GEMM whose bounded waits ran out leaves a 1 in its model's error word (its results are then not to be used); read behind
 // every synchronisation of the library stream.
-int* g_gemm_err = nullptr;
-int* g_gemm_err_dev = nullptr;
 int sync_stream() {
     CK(cudaStreamSynchronize(g_stream));
-    if (g_gemm_err && *reinterpret_cast<volatile int*>(g_gemm_err)) {
-        *reinterpret_cast<volatile int*>(g_gemm_err) = 0;
-        return fail("a tensor-core GEMM gave up waiting for its operands");
-    }
+    if (g_err_words.fetch(g_call_word)) return fail("a tensor-core GEMM gave up waiting for its operands");
     return 0;
 }
 
@@ -369,6 +370,7 @@ struct BeamState {
 
 struct Model {
     ti_model_config cfg{};
+    const int err_word = g_err_words.take();
     std::vector<Layer> layers;
     DevBuf<float> tok_emb, out_norm;
     RawTensor raw_lm;
@@ -435,6 +437,7 @@ struct Model {
         if (xchg) cudaFree(xchg);
         if (graph_decode) cudaGraphExecDestroy(graph_decode);
         if (graph_prefill) cudaGraphExecDestroy(graph_prefill);
+        if (err_word) g_err_words.give(err_word);
     }
 };
 
@@ -465,7 +468,9 @@ QWeight* get_qw(ti_qweight_t h) {
 }
 Model* get_model(ti_model_t h) {
     if (h == 0 || h > g_models.size()) return nullptr;
-    return g_models[h - 1].get();
+    Model* m = g_models[h - 1].get();
+    if (m) g_call_word = m->err_word;
+    return m;
 }
 
 int upload(DevBuf<float>& dst, const float* host, size_t n) {
@@ -1133,7 +1138,7 @@ int launch_step(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args
 struct PairLaunch { CUtensorMap x, w; PairGemmArgs a; int pairs; };
 int pair_gemm_setup(const QWeight& w, const int8_t* planes, const GemmArgs& g, PairLaunch* out) {
     const int n_tiles = (g.N + 2 * kGemmBN - 1) / (2 * kGemmBN), KB = g.k_pad / kGemmBK, pairs = g_num_sms / 2;
-    out->a = PairGemmArgs{g, i8_tile_tokens(g.M, n_tiles, KB, pairs), 0, 0, g_gemm_err_dev};
+    out->a = PairGemmArgs{g, i8_tile_tokens(g.M, n_tiles, KB, pairs), 0, 0, call_err()};
     out->a.tiles_t = (g.M + out->a.T - 1) / out->a.T;
     out->a.tiles = out->a.tiles_t * n_tiles;
     out->pairs = std::min(out->a.tiles, pairs);
@@ -1196,7 +1201,7 @@ int gemm_q_dev(QWeight& w, const float* x_dev, float* y_dev, int M, float* kerne
 int launch_small_gemm(Model& m, QWeight& w, const GemmArgs& g) {
     const int tiles = (w.L.N + kGemmBN - 1) / kGemmBN, KB = w.k_pad / kGemmBK, ctas = small_gemm_ctas(tiles * KB, g_num_sms);
     if (m.pf_ws.n < (size_t)2 * ctas * kSmallRows * kGemmBN || m.pf_cnt.n < (size_t)tiles) return fail("internal: few-row GEMM workspace too small");
-    const SmallArgs sk{reinterpret_cast<const uint8_t*>(m.pf_planes.p), m.pf_ws.p, m.pf_cnt.p, tiles, KB, g_gemm_err_dev};
+    const SmallArgs sk{reinterpret_cast<const uint8_t*>(m.pf_planes.p), m.pf_ws.p, m.pf_cnt.p, tiles, KB, call_err()};
     if (small_rows(g.M) == 16) return launch_step(gemm_i8_tc_small_kernel<16>, dim3(ctas), dim3(kSmallThreads), kSmallSmemBytes, g, sk);
     return launch_step(gemm_i8_tc_small_kernel<32>, dim3(ctas), dim3(kSmallThreads), kSmallSmemBytes, g, sk);
 }
@@ -1275,7 +1280,7 @@ int prefill_attention(Model& m, const float* k_pool, const float* v_pool, const 
         const PrefillKeys keys{k_pool, v_pool, pr.tables, pr.pages_per_seq, m.page_tokens, H, DH, DH, pr.P, kt, h0};
         const PrefillAttn shape{m.pf_qkv.p, m.pf_attn.p, pr.n_seq, pr.P, kt, H, DH, DH, 1, h0, scale};
         kv_images_kernel<DH, DH, PrefillKeys><<<dim3(tiles, nh), 256, 0, g_stream>>>(keys, m.pf_images.p);
-        attn_tc_kernel<DH, DH, PrefillAttn><<<dim3(nh, pr.n_seq * ((pr.P + kAtQ - 1) / kAtQ)), kAtThreads, attn_tc_smem_bytes5<DH, DH>(), g_stream>>>(shape, m.pf_images.p, g_gemm_err_dev);
+        attn_tc_kernel<DH, DH, PrefillAttn><<<dim3(nh, pr.n_seq * ((pr.P + kAtQ - 1) / kAtQ)), kAtThreads, attn_tc_smem_bytes5<DH, DH>(), g_stream>>>(shape, m.pf_images.p, call_err());
         g_launches += 2;
     }
     return 0;
@@ -1786,10 +1791,12 @@ int ti_b200_init(int device) {
     if (prop.major < 10) return fail("ti_b200_init: device %d is sm_%d%d; this library is built for sm_100a (B200) only", device, prop.major, prop.minor);
     g_num_sms = prop.multiProcessorCount;
     if (!g_stream) CK(cudaStreamCreateWithFlags(&g_stream, cudaStreamNonBlocking));
-    if (!g_gemm_err) {
-        CK(cudaHostAlloc(&g_gemm_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-        *g_gemm_err = 0;
-        CK(cudaHostGetDevicePointer(&g_gemm_err_dev, g_gemm_err, 0));
+    if (!g_err_words.host) {
+        int* words = nullptr;
+        CK(cudaHostAlloc(&words, ErrWords::kWords * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        memset(words, 0, ErrWords::kWords * sizeof(int));
+        CK(cudaHostGetDevicePointer(&g_err_words.dev, words, 0));
+        g_err_words.host = words;
     }
     if (g_stage.open() != cudaSuccess) cudaGetLastError();   // (logits then take the driver's own way)
     g_device = device;
