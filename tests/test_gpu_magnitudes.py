@@ -30,10 +30,20 @@ def load(meta, sizes, qt="Q_INT8"):
 
 @pytest.mark.parametrize("sizes", SIZES, ids=str)
 @pytest.mark.parametrize("heads,hidden", [(2, 128), (1, 128), (3, 120)])   # heads of 64, 128 and 40
-@pytest.mark.parametrize("n", [6, 33, 34, 70, 150])   # 5, 32, 33, 69 and 149 common tokens
+@pytest.mark.parametrize("n", [6, 17, 18, 34, 70, 150])   # 5, 16, 17, 33, 69 and 149 common tokens
 def test_common_part_of_a_batch(monkeypatch, sizes, heads, hidden, n):
+    common_part(monkeypatch, sizes, heads, hidden, n, 3)
+
+
+@pytest.mark.parametrize("batch", [1, 2])
+@pytest.mark.parametrize("n", [3, 4])
+def test_two_common_tokens(monkeypatch, batch, n):
+    common_part(monkeypatch, (0, 0, 0), 2, 128, n, batch)
+
+
+def common_part(monkeypatch, sizes, heads, hidden, n, batch):
     meta = dict(vocab=160, hidden=hidden, layers=2, heads=heads, inter=256)
-    prompts = [prompt_tokens(n, meta["vocab"], offset=3 * b) for b in range(3)]
+    prompts = [prompt_tokens(n, meta["vocab"], offset=3 * b) for b in range(batch)]
     m = load(meta, sizes)
     toks, logits, _ = m.generate_batch_greedy(np.array(prompts, dtype=np.int32), 3, want_logits=True)
     monkeypatch.setenv("TURBOINFER_B200_PREFILL", "decode")

@@ -2846,10 +2846,7 @@ static int batch_carveout() {
     return 0;
 }
 
-// rows of a batch's prompts in front of its lockstep steps from which they go through the layers at once (a step needs the byte copy of the
-// weights anyway)
-constexpr int kBatchPromptRows = 6;
-// ... as many rows a pass at most: half a GB of scratch on layers of 4096 (32 prompts of 129 tokens on four of them, us at 1024 / 2048 / 4096 rows: 10977 / 10566 / 10537)
+// rows of a batch's prompts that go through the layers in one pass, at most: half a GB of scratch on layers of 4096 (32 prompts of 129 tokens on four of them, us at 1024 / 2048 / 4096 rows: 10977 / 10566 / 10537)
 constexpr int kBatchPassRows = 2048;
 static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32_t* lens, int32_t batch, int32_t max_len, int32_t n_new,
                                int32_t* out_tokens, float* logits_last, float* decode_ms) {
@@ -2904,10 +2901,11 @@ static int generate_batch_impl(ti_model_t h, const int32_t* prompts, const int32
     }
     BatchState& bs = *m.batch;
     // The prompts' common part -- all tokens in front of the shortest prompt's last one -- goes through the layers at once, as many sequences at a
-    // time as make kBatchPassRows rows; the lockstep steps begin behind it.  (32 prompts of 6 tokens on four 7B-wide layers: five steps of 0.6 ms.)
-    // Rows there is no room for are halved, and without room for one sequence's the steps do it all, with the scratch of a step.
+    // time as make kBatchPassRows rows; the lockstep steps begin behind it.  A pass costs about a step and takes the place of as many as there are common
+    // tokens, from two on (whole calls on four layers, us, with | without: two prompts of 3 tokens 763 | 1032 at 4096 wide, 548 | 728 at 2048; of 4
+    // tokens 757 | 1353 and 548 | 953).  Rows there is no room for are halved, and without room for one sequence's the steps do it all, with the scratch of a step.
     int done = 0;
-    if (min_len > 2 && B * (min_len - 1) >= kBatchPromptRows && prefill_gemm_possible(m)) {
+    if (min_len > 2 && prefill_gemm_possible(m)) {
         const int P = min_len - 1;
         int per = std::max(1, std::min(B, kBatchPassRows / P));
         bool room = false;

@@ -449,8 +449,9 @@ struct SmallArgs {
 };
 // first unit of CTA c (units * CTAs fits 32 bits: at most 2^22 units on 148 SMs)
 TIB_HD int small_unit(int units, int c, int ctas) { return (int)((uint32_t)units * (uint32_t)c / (uint32_t)ctas); }
-// CTAs of a launch: all SMs as long as each has at least four k-steps, a
-// shorter run would be mostly the fix-up of its shared tiles.  Chosen, not swept: only matrices below 592 units (9.7 M weights) are concerned
+// CTAs of a launch: all SMs as long as each has at least four k-steps, a shorter run would be mostly the fix-up of its shared tiles.  Only matrices below 592
+// units (9.7 M weights) are concerned.  A whole step of 4 rows through eight layers, us, at 1 / 2 / 4 / 8 / 16 k-steps: 256 wide 315 / 233 / 304 / 351 / 386, 512 wide
+// 355 / 332 / 272 / 297 / 382, 768 wide 433 / 360 / 412 / 388 / 363, 1024 wide 510 / 413 / 349 / 302 / 336 (best where a run is a whole tile)
 inline int small_gemm_ctas(int units, int sms) { return std::max(1, std::min(sms, units / 4)); }
 
 template <int R>

@@ -587,8 +587,10 @@ __global__ void __launch_bounds__(256) gemv_rows_mma_kernel(const float* A, int 
     };
     const size_t slice = c_end > c_begin ? (size_t)(c_end - c_begin) * 64 : 0;
     // A block's later tiles are asked for two turns ahead, so that memory stays busy while the rows are staged, over the sums at a tile's end and
-    // under the kernel in front; only where the three tiles of all blocks stay in L2 (3 x 40 MB), and where it is known which tiles are read
-    // (one request a step through layers of 2048, a whole answer: 11971 -> 11148 us; four requests: 6451 -> 6217)
+    // under the kernel in front; only where the three tiles of all blocks stay in L2 (3 x 40 MB; limits of 10 to 200 MB: equal), and where it is known
+    // which tiles are read.  Measured, us, built without this | with it: an answer of one request through layers of 2048 11950 | 11200, a step of one row
+    // through two attention layers 2048 wide 160 | 147, 4096 wide 302 | 279, of four rows 191 | 180 and 425 | 408.  (Built with it and the requests
+    // switched off: 11020, 150, 279, 181, 406 -- most of the gain is the loop that the compiler makes of it.)
     const bool ahead = !skip && !nskips && (size_t)gridDim.x * kMmaCols * K * 2 * (GLU ? 2 : 1) <= ((size_t)40 << 20);
     {   // (what the step's rows chose is not known yet: nothing of the experts is asked for)
         const bool expert_tile = nskips && (int)blockIdx.x * kMmaCols >= nskip.first && (int)blockIdx.x * kMmaCols < nskip.first + nskip.group * nskip.count;

@@ -19,7 +19,8 @@ namespace tib {
 namespace seq {
 
 constexpr int kWkvChunk = 16, kWkvCols = 16;
-// rows of a portion from which the chunked form is taken (below it, one launch of the token-by-token scan is as fast)
+// rows of a portion from which the chunked form is taken (a step through two layers of 2048, us, in chunks | token by token: 48 rows 234 | 230, 64 rows
+// 236 | 236, 96 rows 244 | 245, 128 rows 251 | 255, 256 rows 279 | 296)
 constexpr int kWkvChunkedMinRows = 64;
 
 struct WkvChunkArgs {
