@@ -430,7 +430,7 @@ def main():
         wb, kb = model.step_bytes(n_prompt + n_new // 2)
         step_gbs = (wb + kb) * value / seqs / 1e9   # per GPU (step_bytes counts this rank's shards)
         traffic = None
-        for name in ("r02_ncu_decode_kernel_summary.json", "r01_ncu_decode_kernel_summary.json"):
+        for name in ("b_ncu_decode_kernel_summary.json", "a_ncu_decode_kernel_summary.json"):
             try:
                 with open(os.path.join(ROOT, "profiles", name)) as f:
                     traffic = json.load(f).get(workload, {}).get("dram_bytes_per_launch")

@@ -19,9 +19,9 @@
 //                shift of its own accumulator undoes exactly); the B operand's 8 columns carry the three digit planes
 //                (5 columns idle: the tensor pipe has >10x headroom here).  Integer accumulation is exact and order-
 //                independent, so the result does not depend on how k is split over warps or (tensor-parallel) GPUs.
-//                B200 measurement (scripts/microbench5.cu): the integer MMA issues every ~2-3 cycles per SM; the loop runs at
+//                B200 measurement: the integer MMA issues every ~2-3 cycles per SM; the loop runs at
 //                9 cycles per 512-byte item per SM out of shared memory (bound by the shared-memory wavefronts) = 2.4x the HBM
-//                rate.  The IDP4A loop it replaces needed 19-27 (scripts/microbench2/3.cu), the fp32 unpack before 18+.
+//                rate.  The IDP4A loop it replaces needed 19-27, the fp32 unpack before 18+.
 //     reduction  none across lanes: the C fragment of lane (g, t) already holds the sums of columns g, g+8 for digit
 //                planes 2t, 2t+1; one shared-memory integer atomic per (column, digit) when a warp leaves a group
 //   epilogue                    per column: y = colscale * s_x * (A2*65536 + A1*256 + A0 - off*sum(xf) [+ zero-point
@@ -177,7 +177,7 @@ __device__ __forceinline__ void kitem_mma(QuadAcc<BITS>& acc, int par, const uin
 // B fragment of one k-item.  Only B columns 0..2 carry digit planes (lanes g = lane >> 2 < 3); the other lanes read plane 0
 // again (their product columns are never used).  Predicating those lanes off would halve the wavefronts of this load, but
 // costs four register clears per load pair in a loop that is bound by issue slots, not by shared-memory bandwidth: measured
-// slower (profiles/r02_*), so every lane loads.
+// slower (profiles/b_*), so every lane loads.
 template <int BITS>
 __device__ __forceinline__ uint4 load_xfrag(uint32_t addr, bool on) {
     (void)on;
@@ -524,7 +524,7 @@ __device__ __forceinline__ ConsumePlan make_consume_plan(const QLayout& L, const
 // The loop is written for the instruction issue slots: a round is only 4 k-items per warp (4 16-byte loads of weights, 4 of
 // digits, 8 integer MMAs and -- INT4 -- 32 masks), so every instruction of bookkeeping around them shows: the first version of
 // this loop ran ~170 instructions per round and warp and was issue-bound at 0.8 us per stage with the whole ring already in
-// shared memory (profiles/r02_timeline_*: `rounds`).  Hence: barrier and stage addresses as 32-bit shared-window values
+// shared memory (profiles/b_final_timeline_*: `rounds`).  Hence: barrier and stage addresses as 32-bit shared-window values
 // advanced incrementally, the per-round offset sum (REDUX) only on rounds that can be ragged -- a warp whose quad is not in
 // the slab's last group has only full quads before it, so its offset is 4 * warp items -- and no debug code in the
 // production instance.
@@ -541,7 +541,7 @@ __device__ __forceinline__ void gemv_consume(const GemvArgs& a, const Slab& slab
     // B column g = digit plane g.  Columns 3..7 of the product are never read; their lanes duplicate a plane that is read in
     // the SAME quarter-warp (g = 3 -> plane 2, g >= 4 -> plane 0), so that the extra lanes are pure broadcasts: pointing all of
     // them at plane 0 put planes 0 and 2 -- the same banks -- into one quarter-warp of the LDS.128, a 2-way bank conflict on
-    // every digit load (15 % of the kernel's shared-memory load wavefronts in the ncu capture of profiles/r02_*)
+    // every digit load (15 % of the kernel's shared-memory load wavefronts in the ncu capture of profiles/b_*)
     const uint32_t xlane = smem_u32(sm.xd) + ((g < 3 ? g : (g == 3 ? 2 : 0)) * 4 + t) * (BITS == 4 ? 16 : 8);
     const bool xon = g < 3;
     // lane l < 16 stands for warp l when the stage offsets are summed with one REDUX (ragged rounds only)
