@@ -8,7 +8,7 @@ from helpers import make_model, prompt_tokens
 
 pytestmark = pytest.mark.gpu
 
-# products round their rows to bf16 (2^-9 of a value), a dozen in a row; the attention itself is fp32-accurate
+# products round their rows to bf16 (2^-9 of a value), a dozen in a row; the attention itself is accurate to 2^-22 of a value
 TOL = 12 * 2.0 ** -9
 
 

@@ -1,6 +1,6 @@
 """The few-row products (16 or 32 rows a tile, the weight stream dealt to the SMs in k-steps) where they can go wrong: row counts around a
-tile, inner and outer sizes that end inside a k-step or a tile, short prompts and the common part of a batch's prompts.  Against the decode
-engine, whose products run row by row."""
+tile, inner and outer sizes that end inside a k-step or a tile, the common part of a batch's prompts.  Against the decode engine, whose products
+run row by row (and which reads a single request's prompt of fewer than 33 tokens itself)."""
 import numpy as np
 import pytest
 
@@ -33,6 +33,21 @@ def test_short_prompts_equal_the_decode_engine(monkeypatch, meta, qt):
         m.free()
     for got, want in zip(*out):
         assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+
+
+@pytest.mark.parametrize("qt", ["Q_INT8", "Q_INT4"])
+@pytest.mark.parametrize("meta", [SMALL, WIDE], ids=["small", "wide"])
+def test_common_part_of_one_prompt(monkeypatch, meta, qt):
+    import turboinfer_b200 as tb
+    monkeypatch.setenv("TURBOINFER_B200_PREFILL", "")
+    m = model(meta, getattr(tb, qt))
+    prompts = [prompt_tokens(n, meta["vocab"], offset=n) for n in (3, 6, 7, 16, 17, 18, 32, 33, 34)]   # 2 .. 33 rows at once
+    got = [m.generate_batch_greedy(np.array([p], dtype=np.int32), 1, want_logits=True)[1][0] for p in prompts]
+    monkeypatch.setenv("TURBOINFER_B200_PREFILL", "decode")
+    want = [m.prefill(p) for p in prompts]
+    m.free()
+    for g, w in zip(got, want):
+        assert np.abs(g - w).max() <= TOL * np.abs(w).max()
 
 
 @pytest.mark.parametrize("qt", ["Q_INT8", "Q_INT4"])

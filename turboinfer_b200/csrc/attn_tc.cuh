@@ -1,7 +1,9 @@
-// attn_tc.cuh -- softmax attention of prompt rows on the 5th-generation tensor cores at fp32 accuracy, shared by the prefill of the
+// attn_tc.cuh -- softmax attention of prompt rows on the 5th-generation tensor cores from split 16-bit operands, shared by the prefill of the
 // quantized decoder and the prompt portions of the layered sequence engine.
 //
-// Every fp32 operand is split into two fp16 halves, x = hi + lo (hi = fp16(x), lo = fp16(x - hi): 22 mantissa bits), and each product is
+// Every fp32 operand is split into two fp16 halves, x = hi + lo (hi = fp16(x), lo = fp16(x - hi)): 22 mantissa bits from magnitudes of about 2^-3 up, below
+// them an absolute error of about 2^-25 (the low half meets fp16's smallest step), infinite above 65504.  Rows that must not lose range or
+// bits against the decode kernels do not come here (capi.cu prefill_gemm).  Each product is
 // lo hi + hi lo + hi hi with fp32 accumulation, the arithmetic of the warp-level kernels in prefill.cuh / seq_attn_tc.cuh that this replaces
 // for head sizes of 64 and 128 (and smaller ones padded with zeros).  Scores, softmax and the running output stay fp32.
 //
