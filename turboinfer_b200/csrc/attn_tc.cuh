@@ -194,13 +194,14 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const Shape s, c
         const uint32_t bytes = 2 * (is_v ? kV : kK), full = smem_u32(is_v ? v_full : k_full), dst = smem_u32(is_v ? Vs : Ks);
         uint64_t* empty = is_v ? v_empty : k_empty;
         const uint8_t* src = rec0 + (is_v ? 2 * kK : 0) + 2 * step;
-        bool ok = true;
-        for (int i = 2; i < n_tiles && ok; ++i, src += step) {   // (the first two tiles were asked for in front of the query tile)
+        int i = min(2, n_tiles);   // (the first two tiles were asked for in front of the query tile)
+        for (; i < n_tiles; ++i, src += step) {
             const int st = i & 1;
-            ok = mbar_wait_bounded(&empty[st], ((i >> 1) - 1) & 1, err);
+            if (!mbar_wait_bounded(&empty[st], ((i >> 1) - 1) & 1, err)) break;
             mbar_expect_tx_if(full + 8 * st, bytes, lead);
             bulk_g2s_if(dst + st * bytes, src, bytes, full + 8 * st, lead);
         }
+        drain_copies(is_v ? v_full : k_full, 2, i & 1, i >> 1, err);
     } else if (warp == 1) {
         reg_dealloc<80>();
         constexpr uint32_t id_s = umma_idesc_f16(kAtQ, kAtKT, 0), id_o = umma_idesc_f16(kAtQ, DV, 1);

@@ -136,6 +136,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     }
     return true;
 }
+// The last thing a producer does: wait (again with a limit) until the copies it asked for have landed, also when it or another role gave up, so that
+// none arrives in shared memory that the block has left.  Stage i was filled uses + 1 times for i < st, uses times otherwise.  (Copies of both blocks of a
+// pair complete on the even one's barriers; the cluster barrier at the exit holds the odd one.)
+__device__ __forceinline__ void drain_copies(uint64_t* full, int stages, int st, int uses, int* err) {
+    for (int i = 0; i < stages; ++i) {
+        const int n = uses + (i < st ? 1 : 0);
+        if (n > 0) mbar_wait_bounded(&full[i], (n - 1) & 1, err);
+    }
+}
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -318,6 +327,7 @@ gemm_i8_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 if (++st == kGemmStages) { st = 0; ++use; }
             }
         }
+        if (rank == 0) drain_copies(full, kGemmStages, st, use, pg.err);
     } else if (warp == 1) {
         if (rank == 0) {
             const uint32_t lead = elect_one();
@@ -503,13 +513,14 @@ gemm_i8_tc_small_kernel(const GemmArgs g, const SmallArgs sk) {
         for (int i = 0; i < ahead; ++i) weights(u0 + i, i);
         pdl_wait_prior_grid();
         for (int i = 0; i < ahead; ++i) digits(u0 + i, i);
-        bool ok = true;
-        for (int u = u0 + ahead, st = 0, use = 1; u < u1 && ok; ++u) {
-            ok = mbar_wait_bounded(&empty[st], (use - 1) & 1, sk.err);
+        int st = ahead % kStages, use = ahead / kStages;
+        for (int u = u0 + ahead; u < u1; ++u) {
+            if (!mbar_wait_bounded(&empty[st], (use - 1) & 1, sk.err)) break;
             weights(u, st);
             digits(u, st);
             if (++st == kStages) { st = 0; ++use; }
         }
+        drain_copies(full, kStages, st, use, sk.err);
     } else if (warp == 8) {
         // A = weights (unsigned nibbles-in-bytes for INT4, signed for INT8); B = all three signed digit planes at once: their rows are
         // contiguous in the stage, so one MMA with N = 3 R fills the three accumulators (columns R d + m)

@@ -171,6 +171,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (++st == kSgStages) { st = 0; ++use; }
             }
         }
+        if (rank == 0) drain_copies(full, kSgStages, st, use, g.err);
     } else if (warp == 1) {
         if (rank == 0) {
             const uint32_t lead = elect_one();
